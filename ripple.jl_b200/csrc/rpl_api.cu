@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "rpl_internal.h"
+#include "rpl_walk.h"
 
 using rpl::Handle;
 
@@ -77,8 +78,7 @@ void free_all(Handle* h) {
     rpl::free_currents(h);
     void* ptrs[] = {h->N, h->A, h->B, h->d_kappa, h->d_phi, h->d_cos, h->d_sin, h->d_weights, h->d_cgx,
                     h->d_cgy, h->d_cgmag, h->d_depth, h->d_coupling, h->d_wind, h->d_diag, h->d_err,
-                    h->d_coef, h->d_tab32, h->d_cell32, h->d_bin32, h->d_U, h->d_spacing, h->d_sxy,
-                    h->d_vel32, h->d_rmax};
+                    h->d_coef, h->d_tab32, h->d_cell32, h->d_bin32, h->d_U, h->d_spacing, h->d_vel, h->d_rmax};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->h_err) cudaFreeHost(h->h_err);
@@ -261,9 +261,7 @@ int rpl_create(const rpl_desc* d, rpl_handle** out) {
     const size_t elem = d->precision == RPL_FP64 ? 8 : 4;
     const int64_t c3 = d->Nx * d->Ny * d->Nk, P = d->Nx * d->Ny, nb = d->Nk * d->Np;
     int64_t need = 3 * units * (int64_t)elem + 16 * c3 * 8 + (d->depth_kind == RPL_DEPTH_FIELD ? (c3 + P) * 8 : 0) +
-                   (4 * P + 2 * (d->Nx + d->Ny)) * 8 + 6 * P * 8 + 8 * nb * 8 +
-                   (d->precision == RPL_FP32 && d->transport == RPL_TRANSPORT_REFRACTION ? units * 4 + 3 * c3 * 4 : 0) +
-                   (d->precision == RPL_FP32 && d->transport == RPL_TRANSPORT_INTRINSIC ? c3 * 4 + units * 4 : 0);
+                   (4 * P + 2 * (d->Nx + d->Ny)) * 8 + 6 * P * 8 + 8 * nb * 8;
     if (d->memory_limit_bytes > 0 && need > d->memory_limit_bytes)
         return fail(RPL_ERR_OOM, "model needs " + std::to_string(need) + " device bytes, above the memory limit of " +
                                      std::to_string(d->memory_limit_bytes));
@@ -398,18 +396,24 @@ int rpl_create(const rpl_desc* d, rpl_handle** out) {
     TRY(dalloc(h, &h->d_coef, 8 * c3));
     TRY(dalloc(h, &h->d_cell32, 8 * P));
     TRY(dalloc(h, &h->d_bin32, 8 * d->Nk));
-    if (d->transport == RPL_TRANSPORT_REFRACTION && rpl::tile32_supported(*h) && !h->force_column_kernel)
-        TRY(dalloc(h, &h->d_sxy, units));  // the two-pass refraction stage of FP32 models
-    const bool intrinsic32 = d->transport == RPL_TRANSPORT_INTRINSIC && rpl::tile32_supported(*h) &&
-                             !h->force_column_kernel;
-    if ((h->d_sxy || intrinsic32) && rpl::xyw_supported(*h) && !h->pass_a_tiles) {
-        // the y-walk x/y kernels: FP32 velocity planes (intrinsic: c_g only) and upwind ratios
-        const bool refract_planes = h->d_sxy != nullptr;
-        TRY(dalloc(h, &h->d_vel32, (refract_planes ? 3 : 1) * c3));
-        // intrinsic stages with the bundle or learned sources run the x/y pass, then the sources: S
-        if (!refract_planes) TRY(dalloc(h, &h->d_sxy, units));
-        h->vel_regions = rpl::xyw_regions(*h);
-        TRY(dalloc(h, &h->d_rmax, 2 * h->vel_regions * d->Nk));
+    if (rpl::walk_supported(*d)) h->walk = rpl::walk_geometry(*d);
+    if (rpl::walk_supported(*d) && !h->force_column_kernel && !(h->pass_a_tiles && rpl::tile32_supported(*h))) {
+        // the two-pass stage: velocity planes (intrinsic: c_g only) and upwind ratios. A model whose memory
+        // limit or device has no room for them takes the kernels that read the coefficient records.
+        h->vel_regions = (int64_t)h->walk.tiles_x * ((d->Ny + h->walk.seg - 1) / h->walk.seg);
+        const int64_t plane = (d->transport == RPL_TRANSPORT_REFRACTION ? 3 : 1) * c3 * (int64_t)elem;
+        const int64_t ratios = 2 * h->vel_regions * d->Nk * 4;
+        if (!(d->memory_limit_bytes > 0 && need + plane + ratios > d->memory_limit_bytes)) {
+            if (cudaMalloc(&h->d_vel, plane) == cudaSuccess &&
+                cudaMalloc((void**)&h->d_rmax, ratios) == cudaSuccess) {
+                h->bytes += plane + ratios;
+            } else {
+                cudaGetLastError();
+                if (h->d_vel) cudaFree(h->d_vel);
+                h->d_vel = nullptr;
+                h->d_rmax = nullptr;
+            }
+        }
     }
     TRY(rpl::launch_coef(*h, s));
     {

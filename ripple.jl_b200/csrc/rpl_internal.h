@@ -80,16 +80,15 @@ struct TileArgs {
     float lscale;
     const float* lrate;
     const unsigned int* lflag;
-    int learned, pass_b_quads;   // pass_b_quads: pass B of SRC 0/3 stages with four kappa bins per lane
+    int learned, pad1;
     const float* lin_rates;  // SourceTermSet rates per cell-bin (state layout) or null
     int j_lo, j_hi;          // rows the stage updates
-    float* sxy;              // two-pass refraction stage: x+y flux sums per cell-bin (state layout), or null
-    // y-walk pass A (rpl_xyw.cu), or null: FP32 planes of U_x, U_y and the c_g magnitude per (i,j,m),
-    // and the per-region upwind ratios
-    const float* ux32;
-    const float* uy32;
-    const float* cgc32;
-    const unsigned int* rmax;
+    float* sxy;              // two-pass stages: x+y flux sums per cell-bin (state layout); may be Nout itself
+};
+
+// Geometry of the y-walk x/y pass (rpl_xyw.cu).
+struct WalkGeom {
+    int L = 0, CX = 0, tiles_x = 0, seg = 0, threads = 0;
 };
 
 // Tile shapes (kappa-pair lanes per cell L, tile TX x TY) compiled into the ensemble kernel; every
@@ -136,10 +135,11 @@ struct Handle {
     float* d_tab32 = nullptr;      // FP32 copies: 4*Np trig, 2*Nk*Np group velocity, 2*Np cos/sin, Nk*Np weights
     float* d_cell32 = nullptr;     // (Nx*Ny) x 8 floats of per-cell wind constants
     float* d_bin32 = nullptr;      // Nk x 8 floats of per-kappa source constants
-    float* d_sxy = nullptr;        // FP32 refraction models: x+y flux sums between the two stage passes
-    float* d_vel32 = nullptr;      // y-walk pass A: FP32 planes U_x, U_y, c_g per (i,j,m) (3 x Nx*Ny*Nk)
-    unsigned int* d_rmax = nullptr;  // y-walk pass A: per region, axis and bin the upwind ratio maxima
+    void* d_vel = nullptr;         // y-walk x/y pass: planes U_x, U_y, c_g per (i,j,m) in the state's type
+                                   // (intrinsic transport: c_g only); null: the model takes other kernels
+    unsigned int* d_rmax = nullptr;  // y-walk x/y pass: per region, axis and bin the upwind ratio maxima
     int64_t vel_regions = 0;
+    WalkGeom walk;
     // learned source (rpl_learned.cu)
     rpl_mlp* learned = nullptr;
     void* d_lx = nullptr;          // (rows x nbins) BF16 features, rows = cells rounded up to 128
@@ -269,19 +269,13 @@ cudaError_t launch_coef_from_U(const Handle& h, cudaStream_t s);
 // d_U -> the caller-order coupling arrays 0-3 of d_coupling, then their gradients (arrays 4-7).
 cudaError_t launch_export_U(const Handle& h, cudaStream_t s);
 
-// ---- y-walk pass A of the FP32 refraction stage (rpl_xyw.cu) ----
-bool xyw_supported(const Handle& h);              // 32-bit offsets within a direction slice
-int xyw_lanes(int64_t Nk);                        // lanes per cell (four kappa bins each)
-int64_t xyw_regions(const Handle& h);             // regions of the upwind ratio table
-// FP32 velocity planes and upwind ratios from d_coef (after every coefficient refresh; no-op without
-// d_vel32).
-cudaError_t launch_vel32(const Handle& h, cudaStream_t s);
-cudaError_t launch_xyw(const TileArgs& a, cudaStream_t s);   // writes a.sxy for rows [j_lo, j_hi)
-// The same x/y pass for intrinsic transport (no currents): S = fx + fy into a.sxy.
-cudaError_t launch_xy_intrinsic(const TileArgs& a, cudaStream_t s);
-// The whole stage of intrinsic transport (no currents) without sources (src 0) or with the SourceTermSet
-// rates (src 3, the tile body's SRC).
-cudaError_t launch_xyi(const TileArgs& a, int src, cudaStream_t s);
+// ---- two-pass stages (rpl_xyw.cu, rpl_ring.cu, rpl_walk.h) ----
+// Velocity planes and upwind ratios from d_coef (after every coefficient refresh; no-op without d_vel).
+cudaError_t launch_vel(const Handle& h, cudaStream_t s);
+// Where a two-pass stage keeps its x/y flux sums: the stage's own output, which the second pass reads and
+// then overwrites element by element, or buffer A where the output is still an input (stage 3 updates N in
+// place, and A is free by then).
+inline void* stage_scratch(const Handle& h, void* Nout) { return Nout == h.N ? h.A : Nout; }
 
 // ---- FP32 tiled stage kernel (rpl_tile32.cu) ----
 bool tile32_supported(const Handle& h);

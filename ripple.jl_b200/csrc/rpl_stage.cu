@@ -26,6 +26,7 @@
 
 #include "rpl_device.cuh"
 #include "rpl_internal.h"
+#include "rpl_walk.h"
 
 namespace rpl {
 
@@ -460,12 +461,31 @@ StageParams make_params(const Handle& h, double dt, int stage) {
     return p;
 }
 
+namespace {
+
+// The two-pass stage (rpl_xyw.cu, rpl_ring.cu); intrinsic transport without the bundle is one pass.
+template <typename T>
+cudaError_t launch_walk(const Handle& h, const StageParams& p, const void* Nin, const void* N0, void* Nout,
+                        cudaStream_t s) {
+    const bool refract = p.transport == RPL_TRANSPORT_REFRACTION, bundle = p.has_wind || p.has_diss;
+    const WalkArgs<T> a = make_walk_args<T>(h, p, Nin, N0, Nout);
+    if (!refract && !bundle) return launch_xy_stage<T>(a, h.walk, s);
+    cudaError_t e = launch_xy_pass<T>(a, h.walk, s);
+    return e == cudaSuccess ? launch_ring<T>(a, p, refract, bundle, s) : e;
+}
+
+}  // namespace
+
 cudaError_t launch_stage(const Handle& h, const StageParams& p, const void* Nin, const void* N0, void* Nout,
                          cudaStream_t s) {
-    if (h.precision == RPL_FP64) return launch_impl<double, false>(h, p, Nin, N0, Nout, nullptr, s);
+    if (h.precision == RPL_FP64) {
+        if (h.d_vel) return launch_walk<double>(h, p, Nin, N0, Nout, s);
+        return launch_impl<double, false>(h, p, Nin, N0, Nout, nullptr, s);
+    }
     // the tile kernel takes the SourceTermSet rates alone, not together with the bundle or the network
     const bool mixed = p.lin_rates && (p.has_wind || p.has_diss || p.learned);
     if (tile32_supported(h) && !h.force_column_kernel && !mixed) return launch_tile32(h, p, Nin, N0, Nout, s);
+    if (h.d_vel) return launch_walk<float>(h, p, Nin, N0, Nout, s);
     return launch_impl<float, false>(h, p, Nin, N0, Nout, nullptr, s);
 }
 

@@ -23,6 +23,7 @@
 #include "rpl_device.cuh"
 #include "rpl_internal.h"
 #include "rpl_src32.cuh"
+#include "rpl_walk.h"
 #include "rpl_weno32.cuh"
 
 namespace rpl {
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(TX * TY * L, MINB) xy_kernel(const TileArgs p)
 // Pass B: one thread per (cell, kappa pair), CPB cells per CTA, no shared memory.
 template <int L, int CPB, int MINB, int SRC>
 __global__ void __launch_bounds__(CPB * L, MINB) kp_kernel(const TileArgs p) {
-    const float* __restrict__ S = p.sxy;
+    const float* S = p.sxy;   // may be Nout: each element is read, then written, by one thread
     const float* __restrict__ Nin = p.Nin;
     const float* N0 = p.N0;
     float* Nout = p.Nout;
@@ -590,176 +591,6 @@ __global__ void __launch_bounds__(CPB * L, MINB) kp_kernel(const TileArgs p) {
     }
 }
 
-// Pass B with four kappa bins per lane (two packed pairs), for stages without the bundle or learned
-// sources (SRC 0 and 3): the pair kernel's arithmetic element for element, with per-lane overhead
-// (shuffles, window bookkeeping, addressing) shared by four bins. The kappa stencil m0-3 .. m0+6 comes
-// from the lanes below and above (three shuffles each, the reference's clamped indices: Nk % 4 == 0, so
-// only the lowest and the highest live lane clamp).
-template <int L, int CPB, int MINB, int SRC>
-__global__ void __launch_bounds__(CPB * L, MINB) kq_kernel(const TileArgs p) {
-    static_assert(SRC == 0 || SRC == 3, "bundle and learned sources use the pair kernel");
-    const float* __restrict__ S = p.sxy;
-    const float* __restrict__ Nin = p.Nin;
-    const float* N0 = p.N0;
-    float* Nout = p.Nout;
-    const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, Np = p.Np;
-    const int64_t slice = (int64_t)Nx * Ny * Nk;
-    const int64_t P = (int64_t)Nx * (p.j_hi - p.j_lo);
-    const int tid = threadIdx.x, l = tid % L;
-    const int64_t cidx = (int64_t)blockIdx.x * CPB + tid / L;
-    const bool live_cell = cidx < P;
-    const int64_t cc = (live_cell ? cidx : P - 1) + (int64_t)Nx * p.j_lo;
-    const int m0 = 4 * l;
-    const bool live = live_cell && m0 < Nk;
-    const int mc = m0 < Nk ? m0 : Nk - 4;
-    const int64_t home = cc * Nk + mc;
-    const double* r0 = p.coef + 8 * home;
-    auto cq = [&](int f) {
-        return Q{make_float2((float)r0[f], (float)r0[8 + f]), make_float2((float)r0[16 + f], (float)r0[24 + f])};
-    };
-    const Q kap = cq(7), Uxx = cq(2), Uxy = cq(3), Uyx = cq(4), Uyy = cq(5);
-    const float* own = Nin + home;
-    auto wr = [&](int n) { return n < 0 ? n + Np : (n >= Np ? n - Np : n); };
-    Q w0 = ldq(own + slice * wr(-3)), w1 = ldq(own + slice * wr(-2)), w2 = ldq(own + slice * wr(-1));
-    Q w3 = ldq(own), w4 = ldq(own + slice * wr(1)), w5 = ldq(own + slice * wr(2)), w6 = ldq(own + slice * wr(3));
-    const float dk_inv = p.dk_inv, dp_inv = p.dp_inv, dt = p.dt, ca = p.a, cb = p.b;
-    auto full = [&](int q) { return q - 2 >= 0 && q + 3 <= Nk - 1; };   // face q|q+1 has its 5-point stencil
-    const bool hlo = full(m0 - 1), ha = full(m0), hb = full(m0 + 1), hc = full(m0 + 2), hd = full(m0 + 3);
-    const bool up = m0 + 4 <= Nk - 1;   // bins above the quad exist (else clamped to the last bin)
-    Q prevF = qz();
-    bool pvx = false, pvy = false, pvz = false, pvw = false, have = false;
-    for (int n = 0; n < Np; ++n) {
-        const int64_t off = slice * n + home;
-        const Q nxt = ldq(own + slice * ((n + 4) % Np));
-        const Q n0v = (p.stage == 1 || !live) ? qz() : ldq(N0 + off);
-        const Q sxy = ldq(S + off);
-        const Q c = w3;
-        const float4 tg = __ldg(p.trig32 + n);
-        auto ckf = [&](float2 kp_, float2 xx, float2 xy, float2 yx, float2 yy) {
-            return mul2(mul2(f2(-1.f), kp_),
-                        add2(add2(mul2(f2(tg.x), xx), mul2(f2(tg.y), add2(yx, xy))), mul2(f2(tg.z), yy)));
-        };
-        auto cpf = [&](float2 xx, float2 xy, float2 yx, float2 yy) {
-            return sub2(add2(mul2(f2(tg.y), sub2(xx, yy)), mul2(f2(tg.z), yx)), mul2(f2(tg.x), xy));
-        };
-        const Q ck = {ckf(kap.a, Uxx.a, Uxy.a, Uyx.a, Uyy.a), ckf(kap.b, Uxx.b, Uxy.b, Uyx.b, Uyy.b)};
-        const Q cp = {cpf(Uxx.a, Uxy.a, Uyx.a, Uyy.a), cpf(Uxx.b, Uxy.b, Uyx.b, Uyy.b)};
-        const float k0 = c.a.x, k1 = c.a.y, k2 = c.b.x, k3 = c.b.y;
-        const float s_m3 = __shfl_sync(FULL, k1, l - 1, L), s_m2 = __shfl_sync(FULL, k2, l - 1, L);
-        const float s_m1 = __shfl_sync(FULL, k3, l - 1, L);
-        const float s_p4 = __shfl_sync(FULL, k0, l + 1, L), s_p5 = __shfl_sync(FULL, k1, l + 1, L);
-        const float s_p6 = __shfl_sync(FULL, k2, l + 1, L);
-        const float km3 = l >= 1 ? s_m3 : k0, km2 = l >= 1 ? s_m2 : k0, km1 = l >= 1 ? s_m1 : k0;
-        const float kp4 = up ? s_p4 : k3, kp5 = up ? s_p5 : k3, kp6 = up ? s_p6 : k3;
-        // upper faces a..d of bins m0..m0+3, each upwinded by its own bin
-        const bool pa = ck.a.x >= 0.f, pb = ck.a.y >= 0.f, pc = ck.b.x >= 0.f, pd = ck.b.y >= 0.f;
-        float2 Fab, Fcd;
-        if (__all_sync(FULL, pa && pb && pc && pd)) {
-            Fab = weno5_2(make_float2(km2, km1), make_float2(km1, k0), make_float2(k0, k1), make_float2(k1, k2),
-                          make_float2(k2, k3));
-            Fcd = weno5_2(make_float2(k0, k1), make_float2(k1, k2), make_float2(k2, k3), make_float2(k3, kp4),
-                          make_float2(kp4, kp5));
-        } else if (__all_sync(FULL, !pa && !pb && !pc && !pd)) {
-            Fab = weno5_2(make_float2(k3, kp4), make_float2(k2, k3), make_float2(k1, k2), make_float2(k0, k1),
-                          make_float2(km1, k0));
-            Fcd = weno5_2(make_float2(kp5, kp6), make_float2(kp4, kp5), make_float2(k3, kp4), make_float2(k2, k3),
-                          make_float2(k1, k2));
-        } else {
-            Fab = weno5_2(make_float2(pa ? km2 : k3, pb ? km1 : kp4), make_float2(pa ? km1 : k2, pb ? k0 : k3),
-                          make_float2(pa ? k0 : k1, pb ? k1 : k2), make_float2(pa ? k1 : k0, pb ? k2 : k1),
-                          make_float2(pa ? k2 : km1, pb ? k3 : k0));
-            Fcd = weno5_2(make_float2(pc ? k0 : kp5, pd ? k1 : kp6), make_float2(pc ? k1 : kp4, pd ? k2 : kp5),
-                          make_float2(pc ? k2 : k3, pd ? k3 : kp4), make_float2(pc ? k3 : k2, pd ? kp4 : k3),
-                          make_float2(pc ? kp4 : k1, pd ? kp5 : k2));
-        }
-        const float Fa = ha ? Fab.x : (pa ? k0 : k1), Fb = hb ? Fab.y : (pb ? k1 : k2);
-        const float Fc = hc ? Fcd.x : (pc ? k2 : k3), Fd = hd ? Fcd.y : (pd ? k3 : kp4);
-        // lower faces: of m0 the lane below's face d (upwinded by bin m0-1), of m0+1..m0+3 the faces
-        // a..c; recomputed in the bin's own orientation where the two bins' signs differ
-        const float upF = __shfl_up_sync(FULL, Fd, 1, L);
-        const bool upP = __shfl_up_sync(FULL, (int)pd, 1, L) != 0;
-        const bool mA0 = m0 >= 1 && upP != pa, mA1 = pa != pb, mB0 = pb != pc, mB1 = pc != pd;
-        float loA0 = upF, loA1 = Fa, loB0 = Fb, loB1 = Fc;
-        if (mA0 || mA1) {
-            const float2 t = weno5_2(make_float2(pa ? km3 : k2, pb ? km2 : k3), make_float2(pa ? km2 : k1, pb ? km1 : k2),
-                                     make_float2(pa ? km1 : k0, pb ? k0 : k1), make_float2(pa ? k0 : km1, pb ? k1 : k0),
-                                     make_float2(pa ? k1 : km2, pb ? k2 : km1));
-            if (mA0) loA0 = hlo ? t.x : (pa ? km1 : k0);
-            if (mA1) loA1 = ha ? t.y : (pb ? k0 : k1);
-        }
-        if (mB0 || mB1) {
-            const float2 t = weno5_2(make_float2(pc ? km1 : kp4, pd ? k0 : kp5), make_float2(pc ? k0 : k3, pd ? k1 : kp4),
-                                     make_float2(pc ? k1 : k2, pd ? k2 : k3), make_float2(pc ? k2 : k1, pd ? k3 : k2),
-                                     make_float2(pc ? k3 : k0, pd ? kp4 : k1));
-            if (mB0) loB0 = hb ? t.x : (pc ? k1 : k2);
-            if (mB1) loB1 = hc ? t.y : (pd ? k2 : k3);
-        }
-        const Q fk = {mul2(make_float2(kflux(m0 == Nk - 1, m0 == 0, ck.a.x, Fa, loA0),
-                                       kflux(m0 + 1 == Nk - 1, false, ck.a.y, Fb, loA1)), f2(dk_inv)),
-                      mul2(make_float2(kflux(m0 + 2 == Nk - 1, false, ck.b.x, Fc, loB0),
-                                       kflux(m0 + 3 == Nk - 1, false, ck.b.y, Fd, loB1)), f2(dk_inv))};
-        // phi faces: the upper from the window, the lower carried from the previous step unless the sign changed
-        const bool qx = cp.a.x >= 0.f, qy = cp.a.y >= 0.f, qz_ = cp.b.x >= 0.f, qw = cp.b.y >= 0.f;
-        Q Fpp;
-        if (__all_sync(FULL, qx && qy && qz_ && qw)) Fpp = qweno(w1, w2, w3, w4, w5);
-        else if (__all_sync(FULL, !qx && !qy && !qz_ && !qw)) Fpp = qweno(w6, w5, w4, w3, w2);
-        else
-            Fpp = {weno5_2(sel2(qx, qy, w1.a, w6.a), sel2(qx, qy, w2.a, w5.a), sel2(qx, qy, w3.a, w4.a),
-                           sel2(qx, qy, w4.a, w3.a), sel2(qx, qy, w5.a, w2.a)),
-                   weno5_2(sel2(qz_, qw, w1.b, w6.b), sel2(qz_, qw, w2.b, w5.b), sel2(qz_, qw, w3.b, w4.b),
-                           sel2(qz_, qw, w4.b, w3.b), sel2(qz_, qw, w5.b, w2.b))};
-        Q Fpm = prevF;
-        if (!have || pvx != qx || pvy != qy) {
-            const float2 t = weno5_2(sel2(qx, qy, w0.a, w5.a), sel2(qx, qy, w1.a, w4.a), sel2(qx, qy, w2.a, w3.a),
-                                     sel2(qx, qy, w3.a, w2.a), sel2(qx, qy, w4.a, w1.a));
-            if (!have || pvx != qx) Fpm.a.x = t.x;
-            if (!have || pvy != qy) Fpm.a.y = t.y;
-        }
-        if (!have || pvz != qz_ || pvw != qw) {
-            const float2 t = weno5_2(sel2(qz_, qw, w0.b, w5.b), sel2(qz_, qw, w1.b, w4.b), sel2(qz_, qw, w2.b, w3.b),
-                                     sel2(qz_, qw, w3.b, w2.b), sel2(qz_, qw, w4.b, w1.b));
-            if (!have || pvz != qz_) Fpm.b.x = t.x;
-            if (!have || pvw != qw) Fpm.b.y = t.y;
-        }
-        prevF = Fpp;
-        pvx = qx;
-        pvy = qy;
-        pvz = qz_;
-        pvw = qw;
-        have = true;
-        const Q fp = {mul2(mul2(cp.a, sub2(Fpp.a, Fpm.a)), f2(dp_inv)), mul2(mul2(cp.b, sub2(Fpp.b, Fpm.b)), f2(dp_inv))};
-        Q G = {mul2(f2(-1.f), add2(add2(sxy.a, fk.a), fp.a)), mul2(f2(-1.f), add2(add2(sxy.b, fk.b), fp.b))};
-        if constexpr (SRC == 3) {   // SourceTermSet rates of this stage, state layout
-            const Q r = ldq(p.lin_rates + off);
-            G = {fma2(r.a, c.a, G.a), fma2(r.b, c.b, G.b)};
-        }
-        auto upd = [&](float2 g, float2 cv, float2 nv) {
-            float2 st = fma2(f2(dt), g, cv);
-            st.x = relu(st.x);
-            st.y = relu(st.y);
-            float2 out = st;
-            if (p.stage != 1) {
-                out = fma2(f2(ca), nv, mul2(f2(cb), st));
-                out.x = relu(out.x);
-                out.y = relu(out.y);
-            }
-            return out;
-        };
-        const Q out = {upd(G.a, c.a, n0v.a), upd(G.b, c.b, n0v.b)};
-        if (live) {
-            if (!isfinite(out.a.x) || !isfinite(out.a.y) || !isfinite(out.b.x) || !isfinite(out.b.y)) atomicOr(p.err, 1u);
-            stq(Nout + off, out);
-        }
-        w0 = w1;
-        w1 = w2;
-        w2 = w3;
-        w3 = w4;
-        w4 = w5;
-        w5 = w6;
-        w6 = nxt;
-    }
-}
-
 // Second pass of an intrinsic stage with the bundle (SRC 1) or the learned (SRC 2) sources, after the
 // y-walk x/y pass stored S = fx + fy: one thread per (cell, kappa pair) walking the phi ring with the
 // cell's wind constants and its bins' constants loaded once; G = -S, the sources and the stage update
@@ -767,7 +598,7 @@ __global__ void __launch_bounds__(CPB * L, MINB) kq_kernel(const TileArgs p) {
 template <int L, int CPB, int MINB, int SRC>
 __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
     static_assert(SRC == 1 || SRC == 2, "bundle or learned sources");
-    const float* __restrict__ S = p.sxy;
+    const float* S = p.sxy;   // may be Nout: each element is read, then written, by one thread
     const float* __restrict__ Nin = p.Nin;
     const float* N0 = p.N0;
     float* Nout = p.Nout;
@@ -874,26 +705,29 @@ __global__ void __launch_bounds__(ENSEMBLE_THREADS, 1)
     }
 }
 
-template <int L, bool REFRACT, int SRC>
+// Fused stage of intrinsic transport (RPL_PASS_A=tiles).
+template <int L, int SRC>
 cudaError_t launch_variant(const TileArgs& a, int tiles, cudaStream_t s) {
     constexpr int TX = Shape<L>::TX, TY = Shape<L>::TY;
     const size_t smem = tile_smem_bytes(L, TX, TY);
-    auto k = tile_kernel<L, TX, TY, Shape<L>::MINB, REFRACT, SRC>;
+    auto k = tile_kernel<L, TX, TY, Shape<L>::MINB, false, SRC>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k<<<tiles, TX * TY * L, smem, s>>>(a);
     return cudaGetLastError();
 }
 
-// Two-pass refraction stage: pass A over the shape's tiles, then pass B over 256-thread CTAs, three CTAs
-// per SM each (24 warps at <= 80 registers).
+// Two-pass refraction stage: pass A (the y-walk, or staged tiles with RPL_PASS_A=tiles), then pass B: the
+// ring walk with four kappa bins per lane without the bundle or learned sources, else (or with
+// RPL_PASS_B=pairs) the pair kernel in 256-thread CTAs.
 template <int L, int SRC>
-cudaError_t launch_split(const TileArgs& a, cudaStream_t s) {
+cudaError_t launch_split(const Handle& h, const StageParams& p, const TileArgs& a, const WalkArgs<float>& w,
+                         cudaStream_t s) {
     constexpr int TX = Shape<L>::TX, TY = Shape<L>::TY, CPB = 256 / L;
-    const int tiles = ((a.Nx + TX - 1) / TX) * ((a.j_hi - a.j_lo + TY - 1) / TY);
     cudaError_t e;
-    if (a.ux32) {   // the y-walk form (rpl_xyw.cu): one reconstruction per face
-        e = launch_xyw(a, s);
+    if (h.d_vel) {
+        e = launch_xy_pass<float>(w, h.walk, s);
     } else {
+        const int tiles = ((a.Nx + TX - 1) / TX) * ((a.j_hi - a.j_lo + TY - 1) / TY);
         const size_t smem = tile_smem_bytes(L, TX, TY);
         auto ka = xy_kernel<L, TX, TY, 3>;
         cudaFuncSetAttribute(ka, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -901,14 +735,8 @@ cudaError_t launch_split(const TileArgs& a, cudaStream_t s) {
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
+    if ((SRC == 0 || SRC == 3) && !h.pass_b_pairs) return launch_ring<float>(w, p, true, false, s);
     const int64_t cells = (int64_t)a.Nx * (a.j_hi - a.j_lo);
-    if constexpr (SRC == 0 || SRC == 3) {
-        if (a.pass_b_quads) {   // four kappa bins per lane: 128-thread CTAs, four per SM
-            constexpr int L4 = L / 2, QPB = 128 / L4;
-            kq_kernel<L4, QPB, 4, SRC><<<(unsigned)((cells + QPB - 1) / QPB), QPB * L4, 0, s>>>(a);
-            return cudaGetLastError();
-        }
-    }
     // the per-cell source constants of the bundle and the learned source need registers: two CTAs per SM
     constexpr int BMINB = (SRC == 1 || SRC == 2) ? 2 : 3;
     kp_kernel<L, CPB, BMINB, SRC><<<(unsigned)((cells + CPB - 1) / CPB), CPB * L, 0, s>>>(a);
@@ -916,27 +744,21 @@ cudaError_t launch_split(const TileArgs& a, cudaStream_t s) {
 }
 
 template <int L>
-cudaError_t launch_L(const Handle& h, const StageParams& p, const TileArgs& a, cudaStream_t s) {
+cudaError_t launch_L(const Handle& h, const StageParams& p, const TileArgs& a, const WalkArgs<float>& w, cudaStream_t s) {
     constexpr int TX = Shape<L>::TX, TY = Shape<L>::TY;
     const int tiles = (int)(((h.desc.Nx + TX - 1) / TX) * ((p.j_hi - p.j_lo + TY - 1) / TY));
-    const bool refract = p.transport == RPL_TRANSPORT_REFRACTION;
     const int src = p.learned ? 2 : ((p.has_wind || p.has_diss) ? 1 : (p.lin_rates ? 3 : 0));
-    if (refract && a.sxy) {
-        if (src == 3) return launch_split<L, 3>(a, s);
-        if (src == 2) return launch_split<L, 2>(a, s);
-        return src ? launch_split<L, 1>(a, s) : launch_split<L, 0>(a, s);
-    }
-    if (refract) {
-        if (src == 3) return launch_variant<L, true, 3>(a, tiles, s);
-        if (src == 2) return launch_variant<L, true, 2>(a, tiles, s);
-        return src ? launch_variant<L, true, 1>(a, tiles, s) : launch_variant<L, true, 0>(a, tiles, s);
+    if (p.transport == RPL_TRANSPORT_REFRACTION) {
+        if (src == 3) return launch_split<L, 3>(h, p, a, w, s);
+        if (src == 2) return launch_split<L, 2>(h, p, a, w, s);
+        return src ? launch_split<L, 1>(h, p, a, w, s) : launch_split<L, 0>(h, p, a, w, s);
     }
     // the y-walk form (rpl_xyw.cu, one reconstruction per face): one pass without the bundle or learned
     // sources; with them the x/y pass stores S and ks_kernel adds the sources per cell (their per-cell
     // constants loaded once per phi ring) and updates
-    if (a.rmax && (src == 0 || src == 3)) return launch_xyi(a, src, s);
-    if (a.rmax && a.sxy && (src == 1 || src == 2)) {
-        cudaError_t e = launch_xy_intrinsic(a, s);
+    if (h.d_vel && (src == 0 || src == 3)) return launch_xy_stage<float>(w, h.walk, s);
+    if (h.d_vel) {
+        cudaError_t e = launch_xy_pass<float>(w, h.walk, s);
         if (e != cudaSuccess) return e;
         constexpr int CPB = 256 / L;
         const int64_t cells = (int64_t)a.Nx * (a.j_hi - a.j_lo);
@@ -945,9 +767,9 @@ cudaError_t launch_L(const Handle& h, const StageParams& p, const TileArgs& a, c
         else ks_kernel<L, CPB, 2, 2><<<blocks, CPB * L, 0, s>>>(a);
         return cudaGetLastError();
     }
-    if (src == 3) return launch_variant<L, false, 3>(a, tiles, s);
-    if (src == 2) return launch_variant<L, false, 2>(a, tiles, s);
-    return src ? launch_variant<L, false, 1>(a, tiles, s) : launch_variant<L, false, 0>(a, tiles, s);
+    if (src == 3) return launch_variant<L, 3>(a, tiles, s);
+    if (src == 2) return launch_variant<L, 2>(a, tiles, s);
+    return src ? launch_variant<L, 1>(a, tiles, s) : launch_variant<L, 0>(a, tiles, s);
 }
 
 }  // namespace
@@ -1000,19 +822,7 @@ TileArgs make_tile_args(const Handle& h, const StageParams& p, const void* Nin, 
     a.lin_rates = static_cast<const float*>(p.lin_rates);
     a.j_lo = (int)p.j_lo;
     a.j_hi = (int)p.j_hi;
-    a.sxy = h.d_sxy;
-    a.pass_b_quads = !h.pass_b_pairs;
-    if (h.d_vel32) {
-        const int64_t c3 = h.desc.Nx * h.desc.Ny * h.desc.Nk;
-        if (h.desc.transport == RPL_TRANSPORT_REFRACTION) {
-            a.ux32 = h.d_vel32;
-            a.uy32 = h.d_vel32 + c3;
-            a.cgc32 = h.d_vel32 + 2 * c3;
-        } else {
-            a.cgc32 = h.d_vel32;   // intrinsic transport: the c_g plane only
-        }
-        a.rmax = h.d_rmax;
-    }
+    a.sxy = (float*)stage_scratch(h, Nout);
     return a;
 }
 
@@ -1027,10 +837,11 @@ int tile_lanes(int64_t Nk) { return Nk <= 8 ? 4 : (Nk <= 16 ? 8 : 16); }
 cudaError_t launch_tile32(const Handle& h, const StageParams& p, const void* Nin, const void* N0, void* Nout,
                           cudaStream_t s) {
     const TileArgs a = make_tile_args(h, p, Nin, N0, Nout);
+    const WalkArgs<float> w = make_walk_args<float>(h, p, Nin, N0, Nout);
     switch (tile_lanes(h.desc.Nk)) {
-        case 4: return launch_L<4>(h, p, a, s);
-        case 8: return launch_L<8>(h, p, a, s);
-        default: return launch_L<16>(h, p, a, s);
+        case 4: return launch_L<4>(h, p, a, w, s);
+        case 8: return launch_L<8>(h, p, a, w, s);
+        default: return launch_L<16>(h, p, a, w, s);
     }
 }
 
