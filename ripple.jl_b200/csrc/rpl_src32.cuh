@@ -51,12 +51,21 @@ __device__ __forceinline__ float wind_rate32(const P& p, const Cell32& c, const 
     return valid ? rate : 0.0f;
 }
 
-// Source tendency of one cell-bin with action a: wind growth (stress-capped) minus whitecapping.
+// Whether bin b of cell c can grow in any direction: Z falls with cos(theta - theta_u), so it is positive in every
+// direction where it is at cos = 1 (the margin covers the roundings). Away from a storm no bin can, and the
+// growth rate's exponential and division are skipped there.
+template <class P>
+__device__ __forceinline__ bool can_grow32(const P& p, const Cell32& c, const Bin32& b) {
+    return c.on > 0.5f && (b.logk + c.logz1) + p.von_karman32 / fmaf(c.ustar, b.invC, p.z_alpha32) < 1e-3f;
+}
+
+// Source tendency of one cell-bin with action a: wind growth (stress-capped) minus whitecapping. `grows`: the
+// bin may grow in this direction (can_grow32 and cos(theta - theta_u) > 0); false leaves the growth out.
 template <class P>
 __device__ __forceinline__ float source32(const P& p, const Cell32& c, const Bin32& b, float cth, float sth,
-                                          float a) {
+                                          float a, bool grows = true) {
     float g = 0.0f;
-    if (p.has_wind) {
+    if (p.has_wind && grows) {
         float cos_tu;
         const float r = wind_rate32(p, c, b, cth, sth, cos_tu);
         g = (p.stress_cap ? r * c.factor : r) * a;

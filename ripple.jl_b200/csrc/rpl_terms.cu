@@ -159,144 +159,211 @@ __global__ void __launch_bounds__(256) terms_kernel(const T* __restrict__ N, Ter
         }
 }
 
-// Two-kernel form for up to 4 terms. terms_cols_kernel (one warp per column): m0, the mean-spectrum
-// integrals and every term's per-cell values (x0, x1), written to tcol[c * n + t]. terms_bins_kernel:
-// one thread per (m, n) bin walking a chunk of columns with its bin's table entries in registers
-// (NT terms, unrolled), the column values read once per warp (all lanes read the same record) and the
-// rates stored coalesced along kappa. The per-bin arithmetic is terms_kernel's.
+// Two-kernel form for up to 4 terms. terms_cols_kernel: m0, the mean-spectrum integrals and every term's
+// per-cell values (x0, x1), written to tcol[c * n + t]. terms_bins_kernel: the rates of every bin from them.
+//
+// terms_cols_kernel: a warp takes COLS consecutive columns, lanes over the kappa bins, so a bin's table entries
+// serve COLS columns; the tables (weights and the three of the first mean-spectrum term) come from shared
+// memory and the directions go AHEAD at a time, AHEAD COLS loads in flight per lane. (With the tables read through
+// L1 behind the streaming loads, which L1 returns in order, and one column per warp: 822 us at
+// 384 x 384 x 32 x 36; reading the action once is 105 us.)
+constexpr int COLS = 4, COL_WARPS = 8, AHEAD = 4;
+
 template <typename T>
-__global__ void __launch_bounds__(256) terms_cols_kernel(const T* __restrict__ N, TermsArgs a, double2* __restrict__ tcol) {
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void __launch_bounds__(32 * COL_WARPS) terms_cols_kernel(const T* __restrict__ N, TermsArgs a, double2* __restrict__ tcol,
+                                                                    int in_smem) {
+    extern __shared__ double s_tab[];   // weights, then three tables of the mean-spectrum term
     const int lane = threadIdx.x & 31;
-    if (c >= a.P) return;  // uniform per warp
-    const int64_t Nk = a.Nk, Np = a.Np, nb = Nk * Np;
-    // the column pass: m0 and the integrals of the first mean-spectrum term together, four independent
-    // partial sums per lane (directions n mod 4) so the loads of four directions are in flight at once
+    const int Nk = (int)a.Nk, Np = (int)a.Np, nb = Nk * Np;
     int tm = -1;
     for (int t = a.n - 1; t >= 0; --t)
         if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM) tm = t;
-    const double* tbm = a.tabs + (int64_t)(tm < 0 ? 0 : tm) * TABS * nb;
-    double m0p[4] = {0.0, 0.0, 0.0, 0.0}, skp[4] = {0.0, 0.0, 0.0, 0.0}, ssp[4] = {0.0, 0.0, 0.0, 0.0},
-           sdp[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int64_t m = lane; m < Nk; m += 32)
-        for (int64_t n0 = 0; n0 < Np; n0 += 4) {
+    const double* tbm = a.tabs + (int64_t)(tm < 0 ? 0 : tm) * TABS * nb + nb;
+    const double *w = a.weights, *tk = tbm, *ts = tbm + nb, *td = tbm + 2 * nb;
+    if (in_smem) {
+        for (int b = threadIdx.x; b < nb; b += 32 * COL_WARPS) {
+            s_tab[b] = w[b];
+            if (tm >= 0) {
+                s_tab[nb + b] = tk[b];
+                s_tab[2 * nb + b] = ts[b];
+                s_tab[3 * nb + b] = td[b];
+            }
+        }
+        __syncthreads();
+        w = s_tab;
+        tk = s_tab + nb;
+        ts = s_tab + 2 * nb;
+        td = s_tab + 3 * nb;
+    }
+    const int64_t groups = (a.P + COLS - 1) / COLS, slice = a.P * Nk;
+    for (int64_t g = (int64_t)blockIdx.x * COL_WARPS + (threadIdx.x >> 5); g < groups; g += (int64_t)gridDim.x * COL_WARPS) {
+        const int64_t c0 = g * COLS;
+        const int nc = (int)min((int64_t)COLS, a.P - c0);
+        double m0[COLS] = {}, sk[COLS] = {}, ss[COLS] = {}, sd[COLS] = {};
+        for (int m = lane; m < Nk; m += 32) {
+            const T* col = N + c0 * Nk + m;
+            for (int n = 0; n < Np; n += AHEAD) {
+                T v[AHEAD][COLS];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int64_t n = n0 + q;
-                if (n < Np) {
-                    const double v = (double)N[(n * a.P + c) * Nk + m];
-                    const int64_t b = m + Nk * n;
-                    m0p[q] += v * a.weights[b];
-                    if (tm >= 0 && v > 0.0) {
-                        skp[q] += v * tbm[nb + b];
-                        ssp[q] += v * tbm[2 * nb + b];
-                        sdp[q] += v * tbm[3 * nb + b];
+                for (int q = 0; q < AHEAD; ++q)
+#pragma unroll
+                    for (int k = 0; k < COLS; ++k)
+                        v[q][k] = n + q < Np ? __ldg(col + slice * (n + q) + (int64_t)min(k, nc - 1) * Nk) : T(0);
+#pragma unroll
+                for (int q = 0; q < AHEAD; ++q) {
+                    const int b = m + Nk * min(n + q, Np - 1);
+                    const double wb = w[b];
+                    if (tm >= 0) {
+                        const double kb = tk[b], sb = ts[b], db = td[b];
+#pragma unroll
+                        for (int k = 0; k < COLS; ++k) {
+                            const double x = (double)v[q][k], xp = v[q][k] > T(0) ? x : 0.0;
+                            m0[k] = fma(x, wb, m0[k]);
+                            sk[k] = fma(xp, kb, sk[k]);
+                            ss[k] = fma(xp, sb, ss[k]);
+                            sd[k] = fma(xp, db, sd[k]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < COLS; ++k) m0[k] = fma((double)v[q][k], wb, m0[k]);
                     }
                 }
             }
         }
-    const double m0 = warp_sum((m0p[0] + m0p[1]) + (m0p[2] + m0p[3]));
-    for (int t = 0; t < a.n; ++t) {
-        const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
-        double x0 = 0.0, x1 = 0.0;
-        switch (a.kind[t]) {
-            case RPL_TERM_EXPONENTIAL_WIND:
-                x0 = rate;
-                break;
-            case RPL_TERM_WAVE_AGE_WIND:
-                x0 = rate;
-                x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
-                break;
-            case RPL_TERM_WHITECAPPING: {
-                const double excess = fmax(m0 / a.p[t][0] - 1.0, 0.0);
-                x0 = rate * pow(excess, a.p[t][1]);
-                break;
-            }
-            default: {  // mean spectrum: x0 = -C_ds (m0 kbar^2)^2 sigmabar, x1 = kbar (0: no dissipation)
-                double sk, ss, sd;
-                if (t == tm) {
-                    sk = (skp[0] + skp[1]) + (skp[2] + skp[3]);
-                    ss = (ssp[0] + ssp[1]) + (ssp[2] + ssp[3]);
-                    sd = (sdp[0] + sdp[1]) + (sdp[2] + sdp[3]);
-                } else {   // a further mean-spectrum term: its own pass
-                    const double* tb = a.tabs + (int64_t)t * TABS * nb;
-                    sk = ss = sd = 0.0;
-                    for (int64_t n = 0; n < Np; ++n)
-                        for (int64_t m = lane; m < Nk; m += 32) {
-                            const double v = (double)N[(n * a.P + c) * Nk + m];
-                            const int64_t b = m + Nk * n;
-                            if (v > 0.0) {
-                                sk += v * tb[nb + b];
-                                ss += v * tb[2 * nb + b];
-                                sd += v * tb[3 * nb + b];
-                            }
-                        }
-                }
-                const double num_k = warp_sum(sk), num_s = warp_sum(ss), den = warp_sum(sd);
-                const double q = a.p[t][3];
-                const double kbar = den > 0.0 ? pow(num_k / den, 1.0 / q) : 0.0;
-                const double sbar = den > 0.0 ? pow(num_s / den, 1.0 / q) : 0.0;
-                if (m0 > 0.0 && kbar > 0.0) {
-                    const double alpha = m0 * kbar * kbar;
-                    x0 = -a.p[t][0] * alpha * alpha * sbar;
-                    x1 = kbar;
-                }
-                break;
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) {
+            m0[k] = warp_sum(m0[k]);
+            if (tm >= 0) {
+                sk[k] = warp_sum(sk[k]);
+                ss[k] = warp_sum(ss[k]);
+                sd[k] = warp_sum(sd[k]);
             }
         }
-        if (lane == 0) tcol[c * a.n + t] = make_double2(x0, x1);
+        for (int t = 0; t < a.n; ++t) {
+            double f0 = 0.0, f1 = 0.0, f2 = 0.0;   // a further mean-spectrum term: its own pass, column by column
+            for (int k = 0; k < nc; ++k) {
+                const int64_t c = c0 + k;
+                double msk = 0.0, mss = 0.0, msd = 0.0, mm0 = 0.0;
+#pragma unroll
+                for (int q = 0; q < COLS; ++q)
+                    if (q == k) {
+                        mm0 = m0[q];
+                        msk = sk[q];
+                        mss = ss[q];
+                        msd = sd[q];
+                    }
+                if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM && t != tm) {
+                    const double* tb = a.tabs + (int64_t)t * TABS * nb;
+                    f0 = f1 = f2 = 0.0;
+                    for (int n = 0; n < Np; ++n)
+                        for (int m = lane; m < Nk; m += 32) {
+                            const double v = (double)N[slice * n + c * Nk + m];
+                            const int b = m + Nk * n;
+                            if (v > 0.0) {
+                                f0 += v * tb[nb + b];
+                                f1 += v * tb[2 * nb + b];
+                                f2 += v * tb[3 * nb + b];
+                            }
+                        }
+                    msk = warp_sum(f0);
+                    mss = warp_sum(f1);
+                    msd = warp_sum(f2);
+                }
+                if (lane != (k & 31)) continue;   // lane k forms column k's values
+                const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
+                double x0 = 0.0, x1 = 0.0;
+                switch (a.kind[t]) {
+                    case RPL_TERM_EXPONENTIAL_WIND:
+                        x0 = rate;
+                        break;
+                    case RPL_TERM_WAVE_AGE_WIND:
+                        x0 = rate;
+                        x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
+                        break;
+                    case RPL_TERM_WHITECAPPING:
+                        x0 = rate * pow_nonneg(fmax(mm0 / a.p[t][0] - 1.0, 0.0), a.p[t][1]);
+                        break;
+                    default: {  // mean spectrum: the rate of bin k is x0 k + x1 k^2 (both 0: no dissipation)
+                        const double q = a.p[t][3];
+                        const double kbar = msd > 0.0 ? pow(msk / msd, 1.0 / q) : 0.0;
+                        const double sbar = msd > 0.0 ? pow(mss / msd, 1.0 / q) : 0.0;
+                        if (mm0 > 0.0 && kbar > 0.0) {
+                            const double alpha = mm0 * kbar * kbar, cs = -a.p[t][0] * alpha * alpha * sbar;
+                            x0 = cs * a.p[t][1] / kbar;
+                            x1 = cs * a.p[t][2] / (kbar * kbar);
+                        }
+                        break;
+                    }
+                }
+                tcol[c * a.n + t] = make_double2(x0, x1);
+            }
+        }
     }
 }
 
+// terms_bins_kernel: one thread per (m, n) bin walking a chunk of columns with its bin's table entries in
+// registers, the chunk's column values in shared memory, the rates stored coalesced along kappa. A linear term
+// is x0 A + x1 B with A, B of the bin; every division of the formulas is in the column values or the tables
+// (911 us with a division per bin in the mean-spectrum term and the column values read through L1, at
+// 384 x 384 x 32 x 36; writing the rates once is 105 us).
 constexpr int TERM_COLS = 128;   // columns per thread in terms_bins_kernel (more on very large grids)
+
+// x^e for x >= 0 by the exponent's class: 0..4 exactly that power, -1 any other.
+__device__ __forceinline__ double pow_class(double x, int cls, double e) {
+    if (cls == 1) return x;
+    const double x2 = x * x;
+    return cls == 2 ? x2 : (cls == 3 ? x2 * x : (cls == 4 ? x2 * x2 : (cls == 0 ? 1.0 : pow(x, e))));
+}
 
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, const double2* __restrict__ tcol, T* __restrict__ R,
                                                          int64_t chunk) {
+    __shared__ double2 s_col[TERM_COLS * NT];
     const int64_t nb = a.Nk * a.Np;
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
+    const int64_t bin = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, b = min(bin, nb - 1);
     const int64_t Nk = a.Nk, m = b % Nk, n = b / Nk;
     const int64_t c0 = (int64_t)blockIdx.y * chunk, c1 = min(c0 + chunk, a.P);
-    double t0[NT], t1[NT], t2[NT];
+    double A[NT], B[NT];
+    int cls[NT];   // -2: a linear term; else the wave-age input's power class
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         const double* tb = a.tabs + (int64_t)t * TABS * nb;
-        t0[t] = tb[b];
-        t1[t] = tb[nb + b];
-        t2[t] = tb[2 * nb + b];
-    }
-    for (int64_t c = c0; c < c1; ++c) {
-        double r = 0.0;
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            const double2 x = __ldg(tcol + c * NT + t);
-            switch (a.kind[t]) {
-                case RPL_TERM_EXPONENTIAL_WIND:
-                    r += x.x * t0[t];
-                    break;
-                case RPL_TERM_WAVE_AGE_WIND: {
-                    const double al = t0[t];
-                    if (al > 0.0) {
-                        const double excess = fmax(x.y * al * t1[t] - a.p[t][0], 0.0);
-                        r += x.x * pow_nonneg(excess, a.p[t][1]) * t2[t];
-                    }
-                    break;
-                }
-                case RPL_TERM_WHITECAPPING:
-                    r -= x.x * t0[t];
-                    break;
-                default: {
-                    const double k = t0[t];
-                    if (x.y > 0.0 && k > 0.0) {
-                        const double ratio = k / x.y;
-                        r -= x.x * (a.p[t][1] * ratio + a.p[t][2] * ratio * ratio);
-                    }
-                    break;
-                }
-            }
+        const double t0 = tb[b];
+        A[t] = t0;
+        B[t] = 0.0;
+        cls[t] = -2;
+        if (a.kind[t] == RPL_TERM_WAVE_AGE_WIND) {
+            // x0 B max(x1 A - threshold, 0)^power, A = alignment / phase speed; a bin off the wind has no growth
+            // whatever the powers (0^0 = 1): B = 0 there
+            A[t] = t0 * tb[nb + b];
+            B[t] = t0 > 0.0 ? tb[2 * nb + b] : 0.0;
+            const double e = a.p[t][1];
+            cls[t] = e >= 0.0 && e <= 4.0 && e == floor(e) ? (int)e : -1;
+        } else if (a.kind[t] == RPL_TERM_WHITECAPPING) {
+            A[t] = -t0;
+        } else if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM) {
+            A[t] = -t0;
+            B[t] = -t0 * t0;
         }
-        R[(n * a.P + c) * Nk + m] = (T)r;
+    }
+    T* out = R + n * a.P * Nk + m;
+    for (int64_t s0 = c0; s0 < c1; s0 += TERM_COLS) {
+        const int cols = (int)min((int64_t)TERM_COLS, c1 - s0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < cols * NT; k += 256) s_col[k] = tcol[s0 * NT + k];
+        __syncthreads();
+        if (bin >= nb) continue;
+#pragma unroll 4
+        for (int k = 0; k < cols; ++k) {
+            double r = 0.0;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const double2 x = s_col[k * NT + t];
+                if (cls[t] == -2) r = fma(x.x, A[t], fma(x.y, B[t], r));
+                else r = fma(x.x * B[t], pow_class(fmax(fma(x.y, A[t], -a.p[t][0]), 0.0), cls[t], a.p[t][1]), r);
+            }
+            out[(s0 + k) * Nk] = (T)r;
+        }
     }
 }
 
@@ -400,9 +467,18 @@ cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s) {
     const unsigned blocks = (unsigned)((a.P * 32 + 255) / 256);
     const bool fp64 = h.precision == RPL_FP64;
     if (h.d_tcol) {   // up to 4 terms: column values, then the bins
-        if (fp64) terms_cols_kernel<double><<<blocks, 256, 0, s>>>((const double*)Nin, a, h.d_tcol);
-        else terms_cols_kernel<float><<<blocks, 256, 0, s>>>((const float*)Nin, a, h.d_tcol);
-        cudaError_t e = cudaGetLastError();
+        const size_t tab = 4 * a.Nk * a.Np * sizeof(double);
+        const int in_smem = tab <= 100 * 1024;   // two CTAs per SM
+        const unsigned cblocks = (unsigned)std::min<int64_t>((a.P + COLS * COL_WARPS - 1) / (COLS * COL_WARPS), 148 * 8);
+        auto cols = [&](auto k, auto* in) {
+            if (in_smem && tab > 48 * 1024) {
+                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab);
+                if (e != cudaSuccess) return e;
+            }
+            k<<<cblocks, 32 * COL_WARPS, in_smem ? tab : 0, s>>>(in, a, h.d_tcol, in_smem);
+            return cudaGetLastError();
+        };
+        cudaError_t e = fp64 ? cols(terms_cols_kernel<double>, (const double*)Nin) : cols(terms_cols_kernel<float>, (const float*)Nin);
         if (e != cudaSuccess) return e;
         const int64_t chunk = std::max<int64_t>(TERM_COLS, (a.P + 65534) / 65535);   // grid.y <= 65535
         const dim3 grid((unsigned)((a.Nk * a.Np + 255) / 256), (unsigned)((a.P + chunk - 1) / chunk));

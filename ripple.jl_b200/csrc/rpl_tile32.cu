@@ -603,6 +603,9 @@ __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
     const float* N0 = p.N0;
     float* Nout = p.Nout;
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, Np = p.Np;
+    extern __shared__ float2 s_cs[];   // the directions' (cos, sin): not behind the streaming loads in L1
+    for (int n = threadIdx.x; n < Np; n += CPB * L) s_cs[n] = __ldg(p.cs32 + n);
+    __syncthreads();
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const int64_t P = (int64_t)Nx * (p.j_hi - p.j_lo);
     const int tid = threadIdx.x, l = tid % L;
@@ -622,16 +625,25 @@ __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
         lrow = p.lrate + cc * ((int64_t)Nk * Np) + mc;
     }
     const float dt = p.dt, ca = p.a, cb = p.b;
+    const bool grow0 = p.has_wind && can_grow32(p, wc, wb0), grow1 = p.has_wind && can_grow32(p, wc, wb1);
+    // the next direction's values are in flight during a direction
+    float2 cn, sn, nn = f2(0.f);
+    auto fetch = [&](int64_t off) {
+        cn = *reinterpret_cast<const float2*>(Nin + off);
+        sn = *reinterpret_cast<const float2*>(S + off);
+        if (p.stage != 1) nn = *reinterpret_cast<const float2*>(N0 + off);
+    };
+    fetch(home);
     for (int n = 0; n < Np; ++n) {
         const int64_t off = slice * n + home;
-        const float2 c = *reinterpret_cast<const float2*>(Nin + off);
-        const float2 sxy = *reinterpret_cast<const float2*>(S + off);
-        const float2 n0v = (p.stage == 1 || !live) ? f2(0.f) : *reinterpret_cast<const float2*>(N0 + off);
+        const float2 c = cn, sxy = sn, n0v = nn;
+        if (n + 1 < Np) fetch(off + slice);
         float2 G = mul2(f2(-1.f), sxy);
         if (plain_src) {
-            const float2 cs = __ldg(p.cs32 + n);
-            G.x += source32(p, wc, wb0, cs.x, cs.y, c.x);
-            G.y += source32(p, wc, wb1, cs.x, cs.y, c.y);
+            const float2 cs = s_cs[n];
+            const bool with = fmaf(cs.x, wc.cu, cs.y * wc.su) > 0.0f;
+            G.x += source32(p, wc, wb0, cs.x, cs.y, c.x, grow0 && with);
+            G.y += source32(p, wc, wb1, cs.x, cs.y, c.y, grow1 && with);
         } else if constexpr (SRC == 2) {  // learned: N * rate, rate = lscale * sinh(network output of bin (m, n))
             const float2 y = __ldg(reinterpret_cast<const float2*>(lrow + (int64_t)n * Nk));
             G = fma2(mul2(c, f2(p.lscale)), make_float2(sinhf(y.x), sinhf(y.y)), G);
@@ -763,8 +775,8 @@ cudaError_t launch_L(const Handle& h, const StageParams& p, const TileArgs& a, c
         constexpr int CPB = 256 / L;
         const int64_t cells = (int64_t)a.Nx * (a.j_hi - a.j_lo);
         const unsigned blocks = (unsigned)((cells + CPB - 1) / CPB);
-        if (src == 1) ks_kernel<L, CPB, 2, 1><<<blocks, CPB * L, 0, s>>>(a);
-        else ks_kernel<L, CPB, 2, 2><<<blocks, CPB * L, 0, s>>>(a);
+        if (src == 1) ks_kernel<L, CPB, 3, 1><<<blocks, CPB * L, a.Np * sizeof(float2), s>>>(a);
+        else ks_kernel<L, CPB, 2, 2><<<blocks, CPB * L, a.Np * sizeof(float2), s>>>(a);
         return cudaGetLastError();
     }
     if (src == 3) return launch_variant<L, 3>(a, tiles, s);
