@@ -715,8 +715,7 @@ static int set_action_impl(Handle* h, const void* N, int32_t dtype, int32_t layo
                 }
         }
     }
-    RPL_CUDA(rpl::launch_scan_nonfinite(*h, h->N, s));
-    int st = check_error_word(h);
+    int st = check_error_word(h);   // the conversion marks values that are not finite
     if (st) {
         cudaMemsetAsync(h->N, 0, n * h->elem, s);
         cudaStreamSynchronize(s);

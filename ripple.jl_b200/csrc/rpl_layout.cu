@@ -5,8 +5,8 @@
 //   c + P*(m + Nk*n),   c = i + Nx*j, P = Nx*Ny.
 // Device layout of the state: kappa fastest, one contiguous spectral column slice per (i,j,n):
 //   (n*P + c)*Nk + m.
-// For each direction bin n this is the transpose of an Nk x P matrix, done in 32 x 32 tiles
-// through shared memory so both sides are read and written in full 128-byte lines.
+// For each direction bin n this is the transpose of an Nk x P matrix, done in tiles through shared memory
+// so both sides are read and written in full lines.
 #include <cuda_runtime.h>
 
 #include "rpl_internal.h"
@@ -15,43 +15,123 @@ namespace rpl {
 
 namespace {
 
-constexpr int TILE = 32, ROWS = 8;
+// Tiles of CT cells x 32 kappa bins through shared memory. Each thread holds all of its tile's loads (eight) in
+// flight before the first is stored: the pass is bound by memory latency (32 x 32 tiles with four loads in
+// flight took 648 us for 448 x 448 x 32 x 36 FP32, 2.9 TB/s; one read and one write of the state are 287 us).
+// VEC: sixteen bytes (four cells) per access on the caller's side, where its rows are 16-byte aligned.
+constexpr int CT = 64, MT = 32, LTHREADS = 256, PAD = 1;
+
+template <typename S> struct Four { S v[4]; };
 
 // src: rows m0 .. m0+mc-1 of slices n0 .. n0+nc-1 in caller layout, starting at (n0, m0)
-// dst: device layout, whole array
-template <typename S, typename D>
-__global__ void to_device_kernel(const S* __restrict__ src, D* __restrict__ dst, int64_t P, int64_t Nk,
-                                 int64_t n0, int64_t m0, int64_t mc, int64_t src_slice_stride) {
-    __shared__ D tile[TILE][TILE + 1];
-    const int64_t c0 = (int64_t)blockIdx.x * TILE, mb = (int64_t)blockIdx.y * TILE;
+// dst: device layout, whole array. err: bit 2 is set where a converted value is not finite.
+template <typename S, typename D, bool VEC>
+__global__ void __launch_bounds__(LTHREADS) to_device_kernel(const S* __restrict__ src, D* __restrict__ dst, int64_t P, int64_t Nk,
+                                 int64_t n0, int64_t m0, int64_t mc, int64_t src_slice_stride, unsigned int* err) {
+    __shared__ D tile[MT][CT + PAD];
+    const int64_t c0 = (int64_t)blockIdx.x * CT, mb = (int64_t)blockIdx.y * MT;
     const int64_t n = n0 + blockIdx.z;
     const S* s = src + (int64_t)blockIdx.z * src_slice_stride;
-    for (int r = threadIdx.y; r < TILE; r += ROWS) {
-        const int64_t m = mb + r, c = c0 + threadIdx.x;
-        if (m < mc && c < P) tile[r][threadIdx.x] = (D)s[m * P + c];
+    const int nm = (int)min((int64_t)MT, mc - mb), nc = (int)min((int64_t)CT, P - c0);
+    bool bad = false;
+    if (VEC) {
+        constexpr int PER = MT * CT / 4 / LTHREADS;
+        Four<S> v[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / (CT / 4), x = (q % (CT / 4)) * 4;
+            if (r < nm && x < nc) {   // P is a multiple of 4: four cells or none
+                const S* at = s + (mb + r) * P + c0 + x;
+                if constexpr (sizeof(S) == 4) {
+                    const float4 f = __ldcs(reinterpret_cast<const float4*>(at));
+                    v[k] = {(S)f.x, (S)f.y, (S)f.z, (S)f.w};
+                } else {
+                    const double2 f = __ldcs(reinterpret_cast<const double2*>(at)), g = __ldcs(reinterpret_cast<const double2*>(at) + 1);
+                    v[k] = {(S)f.x, (S)f.y, (S)g.x, (S)g.y};
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / (CT / 4), x = (q % (CT / 4)) * 4;
+            if (r < nm && x < nc) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const D d = (D)v[k].v[j];
+                    bad |= !isfinite(d);
+                    tile[r][x + j] = d;
+                }
+            }
+        }
+    } else {
+        constexpr int PER = MT * CT / LTHREADS;
+        S v[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / CT, x = q % CT;
+            if (r < nm && x < nc) v[k] = __ldcs(s + (mb + r) * P + c0 + x);
+        }
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / CT, x = q % CT;
+            if (r < nm && x < nc) {
+                const D d = (D)v[k];
+                bad |= !isfinite(d);
+                tile[r][x] = d;
+            }
+        }
     }
-    __syncthreads();
-    for (int r = threadIdx.y; r < TILE; r += ROWS) {
-        const int64_t c = c0 + r, m = mb + threadIdx.x;
-        if (m < mc && c < P) dst[(n * P + c) * Nk + m0 + m] = tile[threadIdx.x][r];
+    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, 2u);
+    D* out = dst + (n * P + c0) * Nk + m0 + mb;
+#pragma unroll
+    for (int k = 0; k < MT * CT / LTHREADS; ++k) {
+        const int q = threadIdx.x + k * LTHREADS, x = q / MT, r = q % MT;
+        if (r < nm && x < nc) out[x * Nk + r] = tile[r][x];
     }
 }
 
-template <typename S, typename D>
-__global__ void from_device_kernel(const S* __restrict__ src, D* __restrict__ dst, int64_t P, int64_t Nk,
+template <typename S, typename D, bool VEC>
+__global__ void __launch_bounds__(LTHREADS) from_device_kernel(const S* __restrict__ src, D* __restrict__ dst, int64_t P, int64_t Nk,
                                    int64_t n0, int64_t m0, int64_t mc, int64_t dst_slice_stride) {
-    __shared__ D tile[TILE][TILE + 1];
-    const int64_t c0 = (int64_t)blockIdx.x * TILE, mb = (int64_t)blockIdx.y * TILE;
+    __shared__ D tile[MT][CT + PAD];
+    const int64_t c0 = (int64_t)blockIdx.x * CT, mb = (int64_t)blockIdx.y * MT;
     const int64_t n = n0 + blockIdx.z;
     D* d = dst + (int64_t)blockIdx.z * dst_slice_stride;
-    for (int r = threadIdx.y; r < TILE; r += ROWS) {
-        const int64_t c = c0 + r, m = mb + threadIdx.x;
-        if (m < mc && c < P) tile[r][threadIdx.x] = (D)src[(n * P + c) * Nk + m0 + m];
+    const int nm = (int)min((int64_t)MT, mc - mb), nc = (int)min((int64_t)CT, P - c0);
+    const S* in = src + (n * P + c0) * Nk + m0 + mb;
+    S v[MT * CT / LTHREADS];
+#pragma unroll
+    for (int k = 0; k < MT * CT / LTHREADS; ++k) {
+        const int q = threadIdx.x + k * LTHREADS, x = q / MT, r = q % MT;
+        if (r < nm && x < nc) v[k] = __ldcs(in + x * Nk + r);
+    }
+#pragma unroll
+    for (int k = 0; k < MT * CT / LTHREADS; ++k) {
+        const int q = threadIdx.x + k * LTHREADS, x = q / MT, r = q % MT;
+        if (r < nm && x < nc) tile[r][x] = (D)v[k];
     }
     __syncthreads();
-    for (int r = threadIdx.y; r < TILE; r += ROWS) {
-        const int64_t m = mb + r, c = c0 + threadIdx.x;
-        if (m < mc && c < P) d[m * P + c] = tile[threadIdx.x][r];
+    if (VEC) {
+#pragma unroll
+        for (int k = 0; k < MT * CT / 4 / LTHREADS; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / (CT / 4), x = (q % (CT / 4)) * 4;
+            if (r < nm && x < nc) {
+                D* at = d + (mb + r) * P + c0 + x;
+                const D* t = &tile[r][x];
+                if constexpr (sizeof(D) == 4) {
+                    __stcs(reinterpret_cast<float4*>(at), make_float4(t[0], t[1], t[2], t[3]));
+                } else {
+                    __stcs(reinterpret_cast<double2*>(at), make_double2(t[0], t[1]));
+                    __stcs(reinterpret_cast<double2*>(at) + 1, make_double2(t[2], t[3]));
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < MT * CT / LTHREADS; ++k) {
+            const int q = threadIdx.x + k * LTHREADS, r = q / CT, x = q % CT;
+            if (r < nm && x < nc) d[(mb + r) * P + c0 + x] = tile[r][x];
+        }
     }
 }
 
@@ -123,12 +203,16 @@ __global__ void export_U_kernel(int64_t P, int Nk, const double* __restrict__ U,
     for (int a = 0; a < 4; ++a) out[a * c3 + x] = U[a * c3 + t];
 }
 
+// Whether the caller's rows of P cells start on 16-byte boundaries.
+bool aligned_rows(const void* p, int64_t P) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && P % 4 == 0; }
+
 template <typename S, typename D>
 cudaError_t to_dev(const void* src, void* dst, const Handle& h, int64_t n0, int64_t nc, int64_t m0, int64_t mc,
                    cudaStream_t s) {
     const int64_t P = h.cells, Nk = h.desc.Nk;
-    dim3 grid((unsigned)((P + TILE - 1) / TILE), (unsigned)((mc + TILE - 1) / TILE), (unsigned)nc);
-    to_device_kernel<S, D><<<grid, dim3(TILE, ROWS), 0, s>>>((const S*)src, (D*)dst, P, Nk, n0, m0, mc, Nk * P);
+    const dim3 grid((unsigned)((P + CT - 1) / CT), (unsigned)((mc + MT - 1) / MT), (unsigned)nc);
+    auto k = aligned_rows(src, P) ? to_device_kernel<S, D, true> : to_device_kernel<S, D, false>;
+    k<<<grid, LTHREADS, 0, s>>>((const S*)src, (D*)dst, P, Nk, n0, m0, mc, Nk * P, h.d_err);
     return cudaGetLastError();
 }
 
@@ -136,8 +220,9 @@ template <typename S, typename D>
 cudaError_t from_dev(const void* src, void* dst, const Handle& h, int64_t n0, int64_t nc, int64_t m0, int64_t mc,
                      cudaStream_t s) {
     const int64_t P = h.cells, Nk = h.desc.Nk;
-    dim3 grid((unsigned)((P + TILE - 1) / TILE), (unsigned)((mc + TILE - 1) / TILE), (unsigned)nc);
-    from_device_kernel<S, D><<<grid, dim3(TILE, ROWS), 0, s>>>((const S*)src, (D*)dst, P, Nk, n0, m0, mc, Nk * P);
+    const dim3 grid((unsigned)((P + CT - 1) / CT), (unsigned)((mc + MT - 1) / MT), (unsigned)nc);
+    auto k = aligned_rows(dst, P) ? from_device_kernel<S, D, true> : from_device_kernel<S, D, false>;
+    k<<<grid, LTHREADS, 0, s>>>((const S*)src, (D*)dst, P, Nk, n0, m0, mc, Nk * P);
     return cudaGetLastError();
 }
 

@@ -20,6 +20,7 @@
 #include <cmath>
 #include <string>
 
+#include "rpl_colvec.cuh"
 #include "rpl_device.cuh"
 #include "rpl_internal.h"
 
@@ -27,8 +28,8 @@ namespace rpl {
 
 namespace {
 
-constexpr int PM_WARPS = 8;     // columns per block of the velocity kernel
-constexpr int PM_MAX_NK = 256;  // per-warp moments in shared memory: 2 * Nk doubles
+constexpr int PM_WARPS = 8;     // warps per block of the velocity kernel
+constexpr int PM_MAX_NK = 256;  // per-warp moments in shared memory
 
 // Overlap tables of one projection column per block (pseudomomentum.jl:68-121):
 //   O[t,s]  = sum_k Qcell(kappa_t) Qcell(kappa_s) / |dz_k|
@@ -80,45 +81,89 @@ __global__ void pm_overlap_kernel(int Nk, int64_t Nz, int kc_max, const double* 
     }
 }
 
-// Doppler velocity of the pseudomomentum (pseudomomentum.jl:316-342), one warp per (i,j) column.
-// N: device layout (n*P + c)*Nk + m. kx, ky: (Nk, Np) first-moment measures, m fastest. O: the overlap
-// table (or the derivative overlap, for dU/dkappa), one Nk x Nk table (per_cell = 0) or one per column.
-// Ux, Uy: c3 doubles each in device order c*Nk + t. A is the arithmetic type: double for FP64 models
-// and for dU/dkappa, float for the per-stage refresh of FP32 models.
-template <typename T, typename A>
+// Doppler velocity of the pseudomomentum (pseudomomentum.jl:316-342), columns by lane vectors (rpl_colvec.cuh).
+// N: device layout (n*P + c)*Nk + m. kx, ky: (Nk, Np) first-moment measures, m fastest. O: the overlap table
+// (or the derivative overlap, for dU/dkappa), one Nk x Nk table (per_cell = 0; an element read from memory
+// serves the warp's columns) or one per column. Ux, Uy: c3 doubles each in device order c*Nk + t. A is the
+// arithmetic type: double for FP64 models and for dU/dkappa, float for the per-stage refresh of FP32 models.
+// One column per warp took 243 us at 384 x 384 x 32 x 36 FP32; reading the state once is 105 us.
+template <typename T, typename A, bool AL, bool SMEM>
 __global__ void __launch_bounds__(PM_WARPS * 32)
 pm_velocity_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* __restrict__ kx,
                    const A* __restrict__ ky, const A* __restrict__ O, int per_cell, double* __restrict__ Ux,
                    double* __restrict__ Uy) {
+    constexpr int VN = ColVec<T>::N, CH = 12;
     extern __shared__ __align__(16) unsigned char pm_smem[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t c = (int64_t)blockIdx.x * PM_WARPS + w;
-    if (c >= P) return;  // uniform per warp; the kernel has no block-wide barrier
-    A* mx = reinterpret_cast<A*>(pm_smem) + (int64_t)w * 2 * Nk;
-    A* my = mx + Nk;
-    for (int s = lane; s < Nk; s += 32) {
-        A ax = 0, ay = 0;
-#pragma unroll 6
-        for (int n = 0; n < Np; ++n) {
-            const A a = (A)N[((int64_t)n * P + c) * Nk + s];
-            ax += a * __ldg(kx + s + (int64_t)Nk * n);
-            ay += a * __ldg(ky + s + (int64_t)Nk * n);
-        }
-        mx[s] = ax;
-        my[s] = ay;
+    const int warp = threadIdx.x >> 5;
+    const int stride = table_stride<T>(Nk), size = stride * Np;
+    A* tab = reinterpret_cast<A*>(pm_smem);
+    if constexpr (SMEM) {
+        stage_table(tab, kx, Nk, Np, stride);
+        stage_table(tab + size, ky, Nk, Np, stride);
+        __syncthreads();
     }
-    __syncwarp();
-    const A* o = per_cell ? O + c * (int64_t)Nk * Nk : O;
-    for (int t = lane; t < Nk; t += 32) {
-        A ux = 0, uy = 0;
-#pragma unroll 8
-        for (int s = 0; s < Nk; ++s) {
-            const A q = __ldg(o + (int64_t)s * Nk + t);
-            ux += q * mx[s];
-            uy += q * my[s];
+    const ColVec<T> v(Nk);
+    // per warp the moments of its columns, x then y: 2 cpw stride
+    A* mom = tab + (SMEM ? 2 * size : 0) + warp * 2 * v.cpw * stride;
+    A* mx = mom + v.col() * stride;
+    A* my = mx + v.cpw * stride;
+    const int64_t slice = P * Nk, groups = (P + v.cpw - 1) / v.cpw;
+    for (int64_t g = (int64_t)blockIdx.x * PM_WARPS + warp; g < groups; g += (int64_t)gridDim.x * PM_WARPS) {
+        const int64_t col = g * v.cpw + v.col(), c = min(col, P - 1);
+        __syncwarp();
+        for (int m0 = v.l * VN; m0 < Nk; m0 += 32 * VN) {
+            const T* p = N + c * Nk + m0;
+            const int left = Nk - 1 - m0;
+            A ax[VN] = {}, ay[VN] = {};
+            for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
+                T f[CH][VN];
+#pragma unroll
+                for (int k = 0; k < CH; ++k)
+                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, f[k]);
+#pragma unroll
+                for (int k = 0; k < CH; ++k) {
+                    if (n0 + k >= Np) break;
+#pragma unroll
+                    for (int q = 0; q < VN; ++q) {
+                        const int at = (n0 + k) * stride + m0 + q, gb = (n0 + k) * Nk + m0 + min(q, left);
+                        const A a = (A)f[k][q];
+                        ax[q] += a * (SMEM ? tab[at] : __ldg(kx + gb));
+                        ay[q] += a * (SMEM ? tab[size + at] : __ldg(ky + gb));
+                    }
+                }
+            }
+            if (v.used) {
+#pragma unroll
+                for (int q = 0; q < VN; ++q) {
+                    mx[m0 + q] = ax[q];
+                    my[m0 + q] = ay[q];
+                }
+            }
         }
-        Ux[c * Nk + t] = (double)ux;
-        Uy[c * Nk + t] = (double)uy;
+        __syncwarp();
+        const A* o = per_cell ? O + c * (int64_t)Nk * Nk : O;
+        for (int t0 = v.l * VN; t0 < Nk; t0 += 32 * VN) {
+            const int left = Nk - 1 - t0;
+            A ux[VN] = {}, uy[VN] = {};
+#pragma unroll 4
+            for (int s = 0; s < Nk; ++s) {
+                const A px = mx[s], py = my[s];
+#pragma unroll
+                for (int q = 0; q < VN; ++q) {
+                    const A w = __ldg(o + s * Nk + t0 + min(q, left));
+                    ux[q] += w * px;
+                    uy[q] += w * py;
+                }
+            }
+            if (v.used && col < P) {
+#pragma unroll
+                for (int q = 0; q < VN; ++q)
+                    if (q <= left) {
+                        Ux[c * Nk + t0 + q] = (double)ux[q];
+                        Uy[c * Nk + t0 + q] = (double)uy[q];
+                    }
+            }
+        }
     }
 }
 
@@ -134,20 +179,32 @@ int overlap_chunk(int Nk) { return std::max(1, std::min(32, 2048 / Nk)); }
 
 }  // namespace
 
+namespace {
+
+template <typename T, typename A>
+cudaError_t pm_velocity(const Handle& h, const void* Nin, const A* moments, const A* overlap, double* U, cudaStream_t s) {
+    const int Nk = (int)h.desc.Nk, Np = (int)h.desc.Np;
+    const int64_t P = h.cells, c3 = P * Nk, nb = (int64_t)Nk * Np;
+    constexpr int VN = ColVec<T>::N;
+    const int stride = table_stride<T>(Nk);
+    const int64_t cpw = 32 / std::min((Nk + VN - 1) / VN, 32);
+    const size_t mom = (size_t)PM_WARPS * 2 * cpw * stride * sizeof(A), tab = 2 * (size_t)stride * Np * sizeof(A);
+    const bool staged = tab + mom <= kTableBytes;
+    auto k = !staged ? pm_velocity_kernel<T, A, false, false>
+                     : (Nk % VN == 0 ? pm_velocity_kernel<T, A, true, true> : pm_velocity_kernel<T, A, false, true>);
+    const size_t smem = mom + (staged ? tab : 0);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(PM_WARPS * cpw)), 148 * 4);
+    k<<<blocks, PM_WARPS * 32, smem, s>>>((const T*)Nin, P, Nk, Np, moments, moments + nb, overlap, h.pm_cols > 1, U, U + c3);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t launch_pm_refresh(Handle& h, const void* Nin, cudaStream_t s, bool with_derivative) {
-    const rpl_desc& d = h.desc;
-    const int Nk = (int)d.Nk, Np = (int)d.Np;
-    const int64_t P = h.cells, c3 = P * Nk;
-    const unsigned blocks = blocks_for(P, PM_WARPS);
-    if (h.precision == RPL_FP64)
-        pm_velocity_kernel<double, double><<<blocks, PM_WARPS * 32, (size_t)PM_WARPS * 2 * Nk * 8, s>>>(
-            (const double*)Nin, P, Nk, Np, h.d_pm_moments, h.d_pm_moments + (int64_t)Nk * Np, h.d_pm_overlap,
-            h.pm_cols > 1, h.d_U, h.d_U + c3);
-    else
-        pm_velocity_kernel<float, float><<<blocks, PM_WARPS * 32, (size_t)PM_WARPS * 2 * Nk * 4, s>>>(
-            (const float*)Nin, P, Nk, Np, h.d_pm_moments32, h.d_pm_moments32 + (int64_t)Nk * Np, h.d_pm_overlap32,
-            h.pm_cols > 1, h.d_U, h.d_U + c3);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = h.precision == RPL_FP64 ? pm_velocity<double, double>(h, Nin, h.d_pm_moments, h.d_pm_overlap, h.d_U, s)
+                                            : pm_velocity<float, float>(h, Nin, h.d_pm_moments32, h.d_pm_overlap32, h.d_U, s);
     if (e != cudaSuccess) return e;
     e = launch_coef_from_U(h, s);
     if (e != cudaSuccess) return e;
@@ -162,22 +219,11 @@ cudaError_t launch_pm_refresh(Handle& h, const void* Nin, cudaStream_t s, bool w
 }
 
 cudaError_t launch_pm_derivative(const Handle& h, cudaStream_t s) {
-    const rpl_desc& d = h.desc;
-    const int Nk = (int)d.Nk, Np = (int)d.Np;
-    const int64_t P = h.cells, c3 = P * Nk;
+    const int64_t Nk = h.desc.Nk, c3 = h.cells * Nk;
     if (!h.pm_ready) return cudaMemsetAsync(h.d_U + 2 * c3, 0, 2 * c3 * sizeof(double), s);
-    const unsigned blocks = blocks_for(P, PM_WARPS);
-    const size_t smem = (size_t)PM_WARPS * 2 * Nk * 8;
-    const double* Od = h.d_pm_overlap + h.pm_cols * (int64_t)Nk * Nk;
-    if (h.precision == RPL_FP64)
-        pm_velocity_kernel<double, double><<<blocks, PM_WARPS * 32, smem, s>>>(
-            (const double*)h.pm_last_in, P, Nk, Np, h.d_pm_moments, h.d_pm_moments + (int64_t)Nk * Np, Od,
-            h.pm_cols > 1, h.d_U + 2 * c3, h.d_U + 3 * c3);
-    else
-        pm_velocity_kernel<float, double><<<blocks, PM_WARPS * 32, smem, s>>>(
-            (const float*)h.pm_last_in, P, Nk, Np, h.d_pm_moments, h.d_pm_moments + (int64_t)Nk * Np, Od,
-            h.pm_cols > 1, h.d_U + 2 * c3, h.d_U + 3 * c3);
-    return cudaGetLastError();
+    const double* Od = h.d_pm_overlap + h.pm_cols * Nk * Nk;
+    return h.precision == RPL_FP64 ? pm_velocity<double, double>(h, h.pm_last_in, h.d_pm_moments, Od, h.d_U + 2 * c3, s)
+                                   : pm_velocity<float, double>(h, h.pm_last_in, h.d_pm_moments, Od, h.d_U + 2 * c3, s);
 }
 
 void free_pm(Handle* h) {

@@ -6,6 +6,9 @@
 
 #include <algorithm>
 
+#include <type_traits>
+
+#include "rpl_colvec.cuh"
 #include "rpl_device.cuh"
 #include "rpl_internal.h"
 #include "rpl_src32.cuh"
@@ -275,119 +278,119 @@ __device__ __forceinline__ void tadd(double& s, double& c, double v) {
     s = t;
 }
 
-// Per-(i,j) moments (moments.jl:33-37,100-123): one warp per column, lanes over the kappa rings
-// (coalesced reads of each direction's kappa column); per lane, FP64 sums of blocks of 4 directions
-// folded into compensated totals, then a fixed-order compensated butterfly over the lanes
-// (deterministic). The error stays within a few units in the last place of the sum of |terms|.
-// ALL = false computes m0 alone (for the total action), with the same arithmetic for m0.
-template <typename T, bool ALL>
-__global__ void __launch_bounds__(256)
-diag_kernel(const T* __restrict__ N, int64_t Nx, int64_t Ny, int64_t Nk, int64_t Np,
-            const double* __restrict__ tabs, double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t P = Nx * Ny;
-    if (c >= P) return;
-    const int64_t nb = Nk * Np;
-    const double* w = tabs;
-    const double* mux = tabs + nb;
-    const double* muy = tabs + 2 * nb;
-    const double* tr = tabs + 3 * nb;
-    double s0 = 0, c0 = 0, sx = 0, cx = 0, sy = 0, cy = 0, st = 0, ct = 0;
-    const int64_t stride = P * Nk;  // between directions
-    const int nk = (int)Nk, np = (int)Np;
-    for (int m = lane; m < nk; m += 32) {
-        const T* p = N + c * Nk + m;
-        // chunks of CH directions: the chunk's loads are issued together (memory-level parallelism), then
-        // its blocks of DB directions are summed with FMAs and each block sum is folded into the
-        // compensated totals, block by block in direction order
-        constexpr int DB = 4, CH = 3 * DB;
-        for (int n0 = 0; n0 < np; n0 += CH, p += CH * stride) {
-            T a[CH];
+// Per-(i,j) moments (moments.jl:33-37,100-123), columns by lane vectors (rpl_colvec.cuh): per lane, FP64 sums of
+// blocks of four products folded into compensated totals, then a fixed-order compensated fold over the column's
+// lanes (deterministic). The error stays within a few units in the last place of the sum of |terms|.
+// ALL = false computes m0 alone (for the total action), with the same arithmetic for m0. One column per warp
+// with the tables read through L1 took 802 us at 448 x 448 x 32 x 36; reading the state once is 143 us and its
+// FP64 work (a conversion, four FMAs and two compensated adds' share per bin) 150 us.
+template <typename T, bool AL, bool ALL, bool SMEM>
+__global__ void __launch_bounds__(256, 2)
+diag_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const double* __restrict__ tabs, double* __restrict__ out) {
+    constexpr int VN = ColVec<T>::N, TAB = ALL ? 4 : 1, DIRS = 4 / VN, CH = 12;   // a block: DIRS directions of VN bins
+    extern __shared__ __align__(16) double s_tab[];
+    const int stride = table_stride<T>(Nk), size = stride * Np, nb = Nk * Np;
+    if constexpr (SMEM) {
 #pragma unroll
-            for (int k = 0; k < CH; ++k) a[k] = n0 + k < np ? p[k * stride] : T(0);
+        for (int k = 0; k < TAB; ++k) stage_table(s_tab + k * size, tabs + k * nb, Nk, Np, stride);
+        __syncthreads();
+    }
+    const ColVec<T> v(Nk);
+    const int64_t slice = P * Nk, groups = (P + v.cpw - 1) / v.cpw;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
+        const int64_t col = g * v.cpw + v.col(), c = min(col, P - 1);
+        double s[TAB] = {}, e[TAB] = {};
+        for (int m0 = v.l * VN; m0 < Nk; m0 += 32 * VN) {
+            const T* p = N + c * Nk + m0;
+            const int left = Nk - 1 - m0;
+            for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
+                T a[CH][VN];
 #pragma unroll
-            for (int q = 0; q < CH; q += DB) {
-                if (n0 + q >= np) break;
-                double b0 = 0.0, bx = 0.0, by = 0.0, bt = 0.0;
-#pragma unroll
-                for (int k = q; k < q + DB; ++k) {
-                    const int b = n0 + k < np ? m + nk * (n0 + k) : m;  // a[k] = 0 past the last direction
-                    const double ak = (double)a[k];
-                    b0 = fma(ak, __ldg(w + b), b0);
-                    if (ALL) {
-                        bx = fma(ak, __ldg(mux + b), bx);
-                        by = fma(ak, __ldg(muy + b), by);
-                        bt = fma(ak, __ldg(tr + b), bt);
-                    }
+                for (int k = 0; k < CH; ++k) {
+                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, a[k]);
                 }
-                tadd(s0, c0, b0);
-                if (ALL) {
-                    tadd(sx, cx, bx);
-                    tadd(sy, cy, by);
-                    tadd(st, ct, bt);
+#pragma unroll
+                for (int k0 = 0; k0 < CH; k0 += DIRS) {
+                    if (n0 + k0 >= Np) break;
+                    double b[TAB] = {};
+#pragma unroll
+                    for (int k = k0; k < k0 + DIRS; ++k) {
+                        if (n0 + k >= Np) break;
+#pragma unroll
+                        for (int t = 0; t < TAB; ++t)
+#pragma unroll
+                            for (int q = 0; q < VN; ++q) {
+                                const double w = SMEM ? s_tab[t * size + (n0 + k) * stride + m0 + q]
+                                                      : (q <= left ? __ldg(tabs + t * nb + (n0 + k) * Nk + m0 + q) : 0.0);
+                                b[t] = fma((double)a[k][q], w, b[t]);
+                            }
+                    }
+#pragma unroll
+                    for (int t = 0; t < TAB; ++t) tadd(s[t], e[t], b[t]);
                 }
             }
         }
-    }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        double so = __shfl_down_sync(0xffffffffu, s0, off), co = __shfl_down_sync(0xffffffffu, c0, off);
-        tadd(s0, c0, so);
-        c0 += co;
-        if (ALL) {
-            so = __shfl_down_sync(0xffffffffu, sx, off), co = __shfl_down_sync(0xffffffffu, cx, off);
-            tadd(sx, cx, so);
-            cx += co;
-            so = __shfl_down_sync(0xffffffffu, sy, off), co = __shfl_down_sync(0xffffffffu, cy, off);
-            tadd(sy, cy, so);
-            cy += co;
-            so = __shfl_down_sync(0xffffffffu, st, off), co = __shfl_down_sync(0xffffffffu, ct, off);
-            tadd(st, ct, so);
-            ct += co;
+        for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+            for (int t = 0; t < TAB; ++t) {
+                const double so = __shfl_down_sync(0xffffffffu, s[t], off), eo = __shfl_down_sync(0xffffffffu, e[t], off);
+                if (v.l + off < v.L) {
+                    tadd(s[t], e[t], so);
+                    e[t] += eo;
+                }
+            }
         }
-    }
-    if (lane == 0) {
-        const double m0 = s0 + c0;
-        out[c] = m0;
-        if (ALL) {
-            const double mx = sx + cx, my = sy + cy, mt = st + ct;
-            out[P + c] = 4.0 * sqrt(m0);
-            out[2 * P + c] = sqrt(m0 == 0.0 ? 0.0 : mt / m0);
-            out[3 * P + c] = atan2(my, mx);
+        if (v.l == 0 && v.used && col < P) {
+            const double m0 = s[0] + e[0];
+            out[c] = m0;
+            if constexpr (ALL) {
+                const double mx = s[1] + e[1], my = s[2] + e[2], mt = s[3] + e[3];
+                out[P + c] = 4.0 * sqrt(m0);
+                out[2 * P + c] = sqrt(m0 == 0.0 ? 0.0 : mt / m0);
+                out[3 * P + c] = atan2(my, mx);
+            }
         }
     }
 }
 
-// Total action = sum_ij m0 dx dy with a compensated, deterministic two-level reduction.
 // Total action: compensated sum over (i,j) of m0(i,j)·Δx(i)·Δy(j), each cell with its own widths
-// (diagnostic_operations.jl:492-503, bulk_statistics.jl:87-91).
-__global__ void total_kernel(const double* __restrict__ m0, int64_t Nx, int64_t P, const double* __restrict__ xsp,
-                             const double* __restrict__ ysp, double* __restrict__ total) {
-    __shared__ double ss[1024], cc[1024];
+// (diagnostic_operations.jl:492-503, bulk_statistics.jl:87-91), deterministic. Block b sums cells b, b + blocks,
+// ... of every 1024 and leaves (sum, compensation) in part; total_kernel with one block and `parts` set adds
+// the parts in order. (One block for all cells took 288 us at 448 x 448.)
+__global__ void __launch_bounds__(256) total_kernel(const double* __restrict__ m0, int64_t Nx, int64_t P, const double* __restrict__ xsp,
+                                                    const double* __restrict__ ysp, double2* __restrict__ part, int parts,
+                                                    double* __restrict__ total) {
+    __shared__ double2 ss[256];
     double s = 0.0, c = 0.0;
-    const int64_t Ny = P / Nx;
-    for (int64_t j = 0; j < Ny; ++j)
-        for (int64_t i = threadIdx.x; i < Nx; i += blockDim.x) kadd(s, c, m0[j * Nx + i] * xsp[i] * ysp[j]);
-    ss[threadIdx.x] = s;
-    cc[threadIdx.x] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double S = 0.0, C = 0.0;
-        for (unsigned k = 0; k < blockDim.x; ++k) {
-            kadd(S, C, ss[k]);
-            C += cc[k];
+    if (parts == 0) {
+        for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < P; t += (int64_t)gridDim.x * 256) {
+            const int64_t j = t / Nx;
+            kadd(s, c, m0[t] * xsp[t - j * Nx] * ysp[j]);
         }
-        *total = S + C;
+    } else {
+        for (int k = threadIdx.x; k < parts; k += 256) {
+            kadd(s, c, part[k].x);
+            c += part[k].y;
+        }
     }
-}
-
-template <typename T>
-__global__ void nonfinite_kernel(const T* __restrict__ x, int64_t n, unsigned int* err) {
-    bool bad = false;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-        bad |= !isfinite(x[t]);
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, 2u);
+    ss[threadIdx.x] = make_double2(s, c);
+    __syncthreads();
+    for (int h = 128; h > 0; h >>= 1) {
+        if (threadIdx.x < h) {
+            double2 a = ss[threadIdx.x];
+            const double2 b = ss[threadIdx.x + h];
+            kadd(a.x, a.y, b.x);
+            a.y += b.y;
+            ss[threadIdx.x] = a;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (parts == 0) part[blockIdx.x] = ss[0];
+        else *total = ss[0].x + ss[0].y;
+    }
 }
 
 inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
@@ -582,32 +585,33 @@ cudaError_t launch_stress_factor(const Handle& h, const void* Nin, cudaStream_t 
 cudaError_t launch_diagnostics(const Handle& h, const void* Nin, cudaStream_t s, bool moments) {
     const rpl_desc& d = h.desc;
     const int64_t P = d.Nx * d.Ny;
-    const unsigned blocks = blocks_for(P * 32, 256);
-    if (h.precision == RPL_FP64) {
-        if (moments)
-            diag_kernel<double, true><<<blocks, 256, 0, s>>>((const double*)Nin, d.Nx, d.Ny, d.Nk, d.Np, h.d_weights,
-                                                             h.d_diag);
-        else
-            diag_kernel<double, false><<<blocks, 256, 0, s>>>((const double*)Nin, d.Nx, d.Ny, d.Nk, d.Np,
-                                                              h.d_weights, h.d_diag);
-    } else {
-        if (moments)
-            diag_kernel<float, true><<<blocks, 256, 0, s>>>((const float*)Nin, d.Nx, d.Ny, d.Nk, d.Np, h.d_weights,
-                                                            h.d_diag);
-        else
-            diag_kernel<float, false><<<blocks, 256, 0, s>>>((const float*)Nin, d.Nx, d.Ny, d.Nk, d.Np, h.d_weights,
-                                                             h.d_diag);
-    }
-    total_kernel<<<1, 1024, 0, s>>>(h.d_diag, d.Nx, P, h.d_spacing, h.d_spacing + d.Nx, h.d_diag + 4 * P);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_scan_nonfinite(const Handle& h, const void* buf, cudaStream_t s) {
-    const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(h.units, 256), 148 * 32);
-    if (h.precision == RPL_FP64)
-        nonfinite_kernel<double><<<blocks, 256, 0, s>>>((const double*)buf, h.units, h.d_err);
-    else
-        nonfinite_kernel<float><<<blocks, 256, 0, s>>>((const float*)buf, h.units, h.d_err);
+    auto go = [&](auto* in, auto all) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+        constexpr bool ALL = decltype(all)::value;
+        const size_t smem = (ALL ? 4 : 1) * (size_t)table_stride<T>((int)d.Nk) * d.Np * 8;
+        const bool al = d.Nk % ColVec<T>::N == 0;
+        auto k = smem > kTableBytes ? diag_kernel<T, false, ALL, false>
+                                    : (al ? diag_kernel<T, true, ALL, true> : diag_kernel<T, false, ALL, true>);
+        const size_t used = smem > kTableBytes ? 0 : smem;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
+        if (e != cudaSuccess) return e;
+        const int64_t cpw = 32 / std::min<int64_t>((d.Nk + ColVec<T>::N - 1) / ColVec<T>::N, 32);
+        const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(8 * cpw)), 148 * 2);
+        k<<<blocks, 256, used, s>>>(in, P, (int)d.Nk, (int)d.Np, h.d_weights, h.d_diag);
+        return cudaGetLastError();
+    };
+    const std::true_type all;
+    const std::false_type m0_only;
+    cudaError_t e;
+    if (h.precision == RPL_FP64) e = moments ? go((const double*)Nin, all) : go((const double*)Nin, m0_only);
+    else e = moments ? go((const float*)Nin, all) : go((const float*)Nin, m0_only);
+    if (e != cudaSuccess) return e;
+    // the partial sums lie behind the total (slot 4P) in the diagnostics buffer of 5P + 8 doubles
+    const int parts = (int)std::min<int64_t>({(P + 1023) / 1024, 592, (P + 6) / 2});
+    double2* part = reinterpret_cast<double2*>(h.d_diag + 4 * P + 2);
+    const double *xs = h.d_spacing, *ys = h.d_spacing + d.Nx;
+    total_kernel<<<parts, 256, 0, s>>>(h.d_diag, d.Nx, P, xs, ys, part, 0, nullptr);
+    total_kernel<<<1, 256, 0, s>>>(h.d_diag, d.Nx, P, xs, ys, part, parts, h.d_diag + 4 * P);
     return cudaGetLastError();
 }
 

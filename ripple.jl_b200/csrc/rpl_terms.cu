@@ -21,8 +21,10 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
+#include "rpl_colvec.cuh"
 #include "rpl_internal.h"
 
 namespace rpl {
@@ -162,141 +164,115 @@ __global__ void __launch_bounds__(256) terms_kernel(const T* __restrict__ N, Ter
 // Two-kernel form for up to 4 terms. terms_cols_kernel: m0, the mean-spectrum integrals and every term's
 // per-cell values (x0, x1), written to tcol[c * n + t]. terms_bins_kernel: the rates of every bin from them.
 //
-// terms_cols_kernel: a warp takes COLS consecutive columns, lanes over the kappa bins, so a bin's table entries
-// serve COLS columns; the tables (weights and the three of the first mean-spectrum term) come from shared
-// memory and the directions go AHEAD at a time, AHEAD COLS loads in flight per lane. (With the tables read through
-// L1 behind the streaming loads, which L1 returns in order, and one column per warp: 822 us at
-// 384 x 384 x 32 x 36; reading the action once is 105 us.)
-constexpr int COLS = 4, COL_WARPS = 8, AHEAD = 4;
-
-template <typename T>
-__global__ void __launch_bounds__(32 * COL_WARPS) terms_cols_kernel(const T* __restrict__ N, TermsArgs a, double2* __restrict__ tcol,
-                                                                    int in_smem) {
-    extern __shared__ double s_tab[];   // weights, then three tables of the mean-spectrum term
-    const int lane = threadIdx.x & 31;
-    const int Nk = (int)a.Nk, Np = (int)a.Np, nb = Nk * Np;
+// terms_cols_kernel: columns by lane vectors (rpl_colvec.cuh), the tables (weights and the three of the first
+// mean-spectrum term) in shared memory. One column per warp with the tables read through L1 took 822 us at
+// 384 x 384 x 32 x 36; reading the action once is 105 us.
+template <typename T, bool AL, bool SMEM>
+__global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict__ N, TermsArgs a, double2* __restrict__ tcol) {
+    constexpr int VN = ColVec<T>::N, CH = 12;
+    extern __shared__ __align__(16) double s_tab[];   // weights, then the three tables of the mean-spectrum term
+    const int Nk = (int)a.Nk, Np = (int)a.Np, nb = Nk * Np, stride = table_stride<T>(Nk), size = stride * Np;
     int tm = -1;
     for (int t = a.n - 1; t >= 0; --t)
         if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM) tm = t;
     const double* tbm = a.tabs + (int64_t)(tm < 0 ? 0 : tm) * TABS * nb + nb;
-    const double *w = a.weights, *tk = tbm, *ts = tbm + nb, *td = tbm + 2 * nb;
-    if (in_smem) {
-        for (int b = threadIdx.x; b < nb; b += 32 * COL_WARPS) {
-            s_tab[b] = w[b];
-            if (tm >= 0) {
-                s_tab[nb + b] = tk[b];
-                s_tab[2 * nb + b] = ts[b];
-                s_tab[3 * nb + b] = td[b];
-            }
-        }
+    if constexpr (SMEM) {
+        stage_table(s_tab, a.weights, Nk, Np, stride);
+        if (tm >= 0)
+            for (int k = 0; k < 3; ++k) stage_table(s_tab + (k + 1) * size, tbm + k * nb, Nk, Np, stride);
         __syncthreads();
-        w = s_tab;
-        tk = s_tab + nb;
-        ts = s_tab + 2 * nb;
-        td = s_tab + 3 * nb;
     }
-    const int64_t groups = (a.P + COLS - 1) / COLS, slice = a.P * Nk;
-    for (int64_t g = (int64_t)blockIdx.x * COL_WARPS + (threadIdx.x >> 5); g < groups; g += (int64_t)gridDim.x * COL_WARPS) {
-        const int64_t c0 = g * COLS;
-        const int nc = (int)min((int64_t)COLS, a.P - c0);
-        double m0[COLS] = {}, sk[COLS] = {}, ss[COLS] = {}, sd[COLS] = {};
-        for (int m = lane; m < Nk; m += 32) {
-            const T* col = N + c0 * Nk + m;
-            for (int n = 0; n < Np; n += AHEAD) {
-                T v[AHEAD][COLS];
+    const ColVec<T> v(Nk);
+    const int64_t slice = a.P * Nk, groups = (a.P + v.cpw - 1) / v.cpw;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    // sum over the column's lanes, complete in its first lane
+    auto fold = [&](double x) {
 #pragma unroll
-                for (int q = 0; q < AHEAD; ++q)
+        for (int off = 16; off > 0; off >>= 1) {
+            const double y = __shfl_down_sync(0xffffffffu, x, off);
+            if (v.l + off < v.L) x += y;
+        }
+        return x;
+    };
+    for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
+        const int64_t col = g * v.cpw + v.col(), c = min(col, a.P - 1);
+        // two partial sums each (even and odd directions)
+        double m0p[2] = {}, skp[2] = {}, ssp[2] = {}, sdp[2] = {};
+        for (int mm = v.l * VN; mm < Nk; mm += 32 * VN) {
+            const T* p = N + c * Nk + mm;
+            const int left = Nk - 1 - mm;
+            for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
+                T f[CH][VN];
 #pragma unroll
-                    for (int k = 0; k < COLS; ++k)
-                        v[q][k] = n + q < Np ? __ldg(col + slice * (n + q) + (int64_t)min(k, nc - 1) * Nk) : T(0);
+                for (int k = 0; k < CH; ++k)
+                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, f[k]);
 #pragma unroll
-                for (int q = 0; q < AHEAD; ++q) {
-                    const int b = m + Nk * min(n + q, Np - 1);
-                    const double wb = w[b];
-                    if (tm >= 0) {
-                        const double kb = tk[b], sb = ts[b], db = td[b];
+                for (int k = 0; k < CH; ++k) {
+                    if (n0 + k >= Np) break;
 #pragma unroll
-                        for (int k = 0; k < COLS; ++k) {
-                            const double x = (double)v[q][k], xp = v[q][k] > T(0) ? x : 0.0;
-                            m0[k] = fma(x, wb, m0[k]);
-                            sk[k] = fma(xp, kb, sk[k]);
-                            ss[k] = fma(xp, sb, ss[k]);
-                            sd[k] = fma(xp, db, sd[k]);
+                    for (int q = 0; q < VN; ++q) {
+                        const int at = (n0 + k) * stride + mm + q, gb = (n0 + k) * Nk + mm + min(q, left);
+                        const double in = SMEM || q <= left ? 1.0 : 0.0;
+                        const double x = (double)f[k][q];
+                        m0p[k & 1] = fma(x, SMEM ? s_tab[at] : in * __ldg(a.weights + gb), m0p[k & 1]);
+                        if (tm >= 0) {
+                            const double xp = f[k][q] > T(0) ? x : 0.0;
+                            skp[k & 1] = fma(xp, SMEM ? s_tab[size + at] : in * __ldg(tbm + gb), skp[k & 1]);
+                            ssp[k & 1] = fma(xp, SMEM ? s_tab[2 * size + at] : in * __ldg(tbm + nb + gb), ssp[k & 1]);
+                            sdp[k & 1] = fma(xp, SMEM ? s_tab[3 * size + at] : in * __ldg(tbm + 2 * nb + gb), sdp[k & 1]);
                         }
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < COLS; ++k) m0[k] = fma((double)v[q][k], wb, m0[k]);
                     }
                 }
             }
         }
-#pragma unroll
-        for (int k = 0; k < COLS; ++k) {
-            m0[k] = warp_sum(m0[k]);
-            if (tm >= 0) {
-                sk[k] = warp_sum(sk[k]);
-                ss[k] = warp_sum(ss[k]);
-                sd[k] = warp_sum(sd[k]);
-            }
-        }
+        const double m0 = fold(m0p[0] + m0p[1]);
+        const double sk = fold(skp[0] + skp[1]), ss = fold(ssp[0] + ssp[1]), sd = fold(sdp[0] + sdp[1]);
         for (int t = 0; t < a.n; ++t) {
-            double f0 = 0.0, f1 = 0.0, f2 = 0.0;   // a further mean-spectrum term: its own pass, column by column
-            for (int k = 0; k < nc; ++k) {
-                const int64_t c = c0 + k;
-                double msk = 0.0, mss = 0.0, msd = 0.0, mm0 = 0.0;
-#pragma unroll
-                for (int q = 0; q < COLS; ++q)
-                    if (q == k) {
-                        mm0 = m0[q];
-                        msk = sk[q];
-                        mss = ss[q];
-                        msd = sd[q];
-                    }
-                if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM && t != tm) {
-                    const double* tb = a.tabs + (int64_t)t * TABS * nb;
-                    f0 = f1 = f2 = 0.0;
-                    for (int n = 0; n < Np; ++n)
-                        for (int m = lane; m < Nk; m += 32) {
-                            const double v = (double)N[slice * n + c * Nk + m];
-                            const int b = m + Nk * n;
-                            if (v > 0.0) {
-                                f0 += v * tb[nb + b];
-                                f1 += v * tb[2 * nb + b];
-                                f2 += v * tb[3 * nb + b];
-                            }
+            double msk = sk, mss = ss, msd = sd;
+            if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM && t != tm) {   // a further mean-spectrum term: its own pass
+                const double* tb = a.tabs + (int64_t)t * TABS * nb;
+                double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+                for (int n = 0; n < Np; ++n)
+                    for (int m = v.l; m < Nk; m += v.L) {
+                        const double x = (double)N[slice * n + c * Nk + m];
+                        const int b = m + Nk * n;
+                        if (x > 0.0) {
+                            f0 += x * tb[nb + b];
+                            f1 += x * tb[2 * nb + b];
+                            f2 += x * tb[3 * nb + b];
                         }
-                    msk = warp_sum(f0);
-                    mss = warp_sum(f1);
-                    msd = warp_sum(f2);
-                }
-                if (lane != (k & 31)) continue;   // lane k forms column k's values
-                const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
-                double x0 = 0.0, x1 = 0.0;
-                switch (a.kind[t]) {
-                    case RPL_TERM_EXPONENTIAL_WIND:
-                        x0 = rate;
-                        break;
-                    case RPL_TERM_WAVE_AGE_WIND:
-                        x0 = rate;
-                        x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
-                        break;
-                    case RPL_TERM_WHITECAPPING:
-                        x0 = rate * pow_nonneg(fmax(mm0 / a.p[t][0] - 1.0, 0.0), a.p[t][1]);
-                        break;
-                    default: {  // mean spectrum: the rate of bin k is x0 k + x1 k^2 (both 0: no dissipation)
-                        const double q = a.p[t][3];
-                        const double kbar = msd > 0.0 ? pow(msk / msd, 1.0 / q) : 0.0;
-                        const double sbar = msd > 0.0 ? pow(mss / msd, 1.0 / q) : 0.0;
-                        if (mm0 > 0.0 && kbar > 0.0) {
-                            const double alpha = mm0 * kbar * kbar, cs = -a.p[t][0] * alpha * alpha * sbar;
-                            x0 = cs * a.p[t][1] / kbar;
-                            x1 = cs * a.p[t][2] / (kbar * kbar);
-                        }
-                        break;
                     }
-                }
-                tcol[c * a.n + t] = make_double2(x0, x1);
+                msk = fold(f0);
+                mss = fold(f1);
+                msd = fold(f2);
             }
+            if (v.l != 0 || !v.used || col >= a.P) continue;
+            const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
+            double x0 = 0.0, x1 = 0.0;
+            switch (a.kind[t]) {
+                case RPL_TERM_EXPONENTIAL_WIND:
+                    x0 = rate;
+                    break;
+                case RPL_TERM_WAVE_AGE_WIND:
+                    x0 = rate;
+                    x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
+                    break;
+                case RPL_TERM_WHITECAPPING:
+                    x0 = rate * pow_nonneg(fmax(m0 / a.p[t][0] - 1.0, 0.0), a.p[t][1]);
+                    break;
+                default: {  // mean spectrum: the rate of bin k is x0 k + x1 k^2 (both 0: no dissipation)
+                    const double q = a.p[t][3];
+                    const double kbar = msd > 0.0 ? pow(msk / msd, 1.0 / q) : 0.0;
+                    const double sbar = msd > 0.0 ? pow(mss / msd, 1.0 / q) : 0.0;
+                    if (m0 > 0.0 && kbar > 0.0) {
+                        const double alpha = m0 * kbar * kbar, cs = -a.p[t][0] * alpha * alpha * sbar;
+                        x0 = cs * a.p[t][1] / kbar;
+                        x1 = cs * a.p[t][2] / (kbar * kbar);
+                    }
+                    break;
+                }
+            }
+            tcol[c * a.n + t] = make_double2(x0, x1);
         }
     }
 }
@@ -308,14 +284,8 @@ __global__ void __launch_bounds__(32 * COL_WARPS) terms_cols_kernel(const T* __r
 // 384 x 384 x 32 x 36; writing the rates once is 105 us).
 constexpr int TERM_COLS = 128;   // columns per thread in terms_bins_kernel (more on very large grids)
 
-// x^e for x >= 0 by the exponent's class: 0..4 exactly that power, -1 any other.
-__device__ __forceinline__ double pow_class(double x, int cls, double e) {
-    if (cls == 1) return x;
-    const double x2 = x * x;
-    return cls == 2 ? x2 : (cls == 3 ? x2 * x : (cls == 4 ? x2 * x2 : (cls == 0 ? 1.0 : pow(x, e))));
-}
-
-template <typename T, int NT>
+// LINEAR_POWER: every wave-age term has power 1 (the reference's default); else pow_nonneg.
+template <typename T, int NT, bool LINEAR_POWER>
 __global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, const double2* __restrict__ tcol, T* __restrict__ R,
                                                          int64_t chunk) {
     __shared__ double2 s_col[TERM_COLS * NT];
@@ -324,21 +294,19 @@ __global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, const doub
     const int64_t Nk = a.Nk, m = b % Nk, n = b / Nk;
     const int64_t c0 = (int64_t)blockIdx.y * chunk, c1 = min(c0 + chunk, a.P);
     double A[NT], B[NT];
-    int cls[NT];   // -2: a linear term; else the wave-age input's power class
+    bool wave_age[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         const double* tb = a.tabs + (int64_t)t * TABS * nb;
         const double t0 = tb[b];
         A[t] = t0;
         B[t] = 0.0;
-        cls[t] = -2;
-        if (a.kind[t] == RPL_TERM_WAVE_AGE_WIND) {
+        wave_age[t] = a.kind[t] == RPL_TERM_WAVE_AGE_WIND;
+        if (wave_age[t]) {
             // x0 B max(x1 A - threshold, 0)^power, A = alignment / phase speed; a bin off the wind has no growth
             // whatever the powers (0^0 = 1): B = 0 there
             A[t] = t0 * tb[nb + b];
             B[t] = t0 > 0.0 ? tb[2 * nb + b] : 0.0;
-            const double e = a.p[t][1];
-            cls[t] = e >= 0.0 && e <= 4.0 && e == floor(e) ? (int)e : -1;
         } else if (a.kind[t] == RPL_TERM_WHITECAPPING) {
             A[t] = -t0;
         } else if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM) {
@@ -359,8 +327,12 @@ __global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, const doub
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 const double2 x = s_col[k * NT + t];
-                if (cls[t] == -2) r = fma(x.x, A[t], fma(x.y, B[t], r));
-                else r = fma(x.x * B[t], pow_class(fmax(fma(x.y, A[t], -a.p[t][0]), 0.0), cls[t], a.p[t][1]), r);
+                if (!wave_age[t]) {
+                    r = fma(x.x, A[t], fma(x.y, B[t], r));
+                } else {
+                    const double excess = fmax(fma(x.y, A[t], -a.p[t][0]), 0.0);
+                    r = fma(x.x * B[t], LINEAR_POWER ? excess : pow_nonneg(excess, a.p[t][1]), r);
+                }
             }
             out[(s0 + k) * Nk] = (T)r;
         }
@@ -467,26 +439,34 @@ cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s) {
     const unsigned blocks = (unsigned)((a.P * 32 + 255) / 256);
     const bool fp64 = h.precision == RPL_FP64;
     if (h.d_tcol) {   // up to 4 terms: column values, then the bins
-        const size_t tab = 4 * a.Nk * a.Np * sizeof(double);
-        const int in_smem = tab <= 100 * 1024;   // two CTAs per SM
-        const unsigned cblocks = (unsigned)std::min<int64_t>((a.P + COLS * COL_WARPS - 1) / (COLS * COL_WARPS), 148 * 8);
-        auto cols = [&](auto k, auto* in) {
-            if (in_smem && tab > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab);
-                if (e != cudaSuccess) return e;
-            }
-            k<<<cblocks, 32 * COL_WARPS, in_smem ? tab : 0, s>>>(in, a, h.d_tcol, in_smem);
+        auto cols = [&](auto* in) {
+            using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+            constexpr int VN = ColVec<T>::N;
+            const size_t smem = 4 * (size_t)table_stride<T>((int)a.Nk) * a.Np * 8, used = smem > kTableBytes ? 0 : smem;
+            auto k = !used ? terms_cols_kernel<T, false, false>
+                           : (a.Nk % VN == 0 ? terms_cols_kernel<T, true, true> : terms_cols_kernel<T, false, true>);
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
+            if (e != cudaSuccess) return e;
+            const int64_t per = 8 * (32 / std::min<int64_t>((a.Nk + VN - 1) / VN, 32));
+            k<<<(unsigned)std::min<int64_t>((a.P + per - 1) / per, 148 * 2), 256, used, s>>>(in, a, h.d_tcol);
             return cudaGetLastError();
         };
-        cudaError_t e = fp64 ? cols(terms_cols_kernel<double>, (const double*)Nin) : cols(terms_cols_kernel<float>, (const float*)Nin);
+        cudaError_t e = fp64 ? cols((const double*)Nin) : cols((const float*)Nin);
         if (e != cudaSuccess) return e;
         const int64_t chunk = std::max<int64_t>(TERM_COLS, (a.P + 65534) / 65535);   // grid.y <= 65535
         const dim3 grid((unsigned)((a.Nk * a.Np + 255) / 256), (unsigned)((a.P + chunk - 1) / chunk));
+        bool linear = true;
+        for (int t = 0; t < a.n; ++t) linear = linear && (a.kind[t] != RPL_TERM_WAVE_AGE_WIND || a.p[t][1] == 1.0);
         switch (a.n) {
 #define RPL_BINS(NT)                                                                                           \
     case NT:                                                                                                   \
-        if (fp64) terms_bins_kernel<double, NT><<<grid, 256, 0, s>>>(a, h.d_tcol, (double*)h.d_lin_rates, chunk); \
-        else terms_bins_kernel<float, NT><<<grid, 256, 0, s>>>(a, h.d_tcol, (float*)h.d_lin_rates, chunk);  \
+        if (fp64) {                                                                                            \
+            if (linear) terms_bins_kernel<double, NT, true><<<grid, 256, 0, s>>>(a, h.d_tcol, (double*)h.d_lin_rates, chunk); \
+            else terms_bins_kernel<double, NT, false><<<grid, 256, 0, s>>>(a, h.d_tcol, (double*)h.d_lin_rates, chunk);       \
+        } else {                                                                                               \
+            if (linear) terms_bins_kernel<float, NT, true><<<grid, 256, 0, s>>>(a, h.d_tcol, (float*)h.d_lin_rates, chunk);   \
+            else terms_bins_kernel<float, NT, false><<<grid, 256, 0, s>>>(a, h.d_tcol, (float*)h.d_lin_rates, chunk);         \
+        }                                                                                                      \
         break;
             RPL_BINS(1)
             RPL_BINS(2)
