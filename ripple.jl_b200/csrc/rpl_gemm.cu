@@ -46,7 +46,8 @@ struct GemmSmem {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE = A_BYTES + B_BYTES;  // a multiple of 1024
-    static constexpr int TOTAL = STAGES * STAGE + 1024 /* alignment slack */;
+    static constexpr int STAGING = EPI_WARPS * 2048;   // per epilogue warp 32 rows x 64 bytes
+    static constexpr int TOTAL = STAGES * STAGE + STAGING + 1024 /* alignment slack */;
 };
 
 // The network's activation: GELU in its tanh form, 0.5 z (1 + tanh(c (z + a z^3))), c = sqrt(2/pi),
@@ -81,75 +82,103 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volati
     return false;
 }
 
-// Fused epilogue of COLS accumulator columns for the thread holding row `row`: reads its TMEM lane
-// starting at TMEM address `trow`, writes output columns n0 .. n0 + COLS - 1.
-template <int COLS, int EPI>
-__device__ __forceinline__ void epilogue_cols(const GemmArgs& g, uint32_t trow, int row, int n0) {
-    float ex[4] = {0.f, 0.f, 0.f, 0.f};
-    if (EPI == EPI_BIAS_GELU && g.extra) {
+// A warp's 32 rows x 64 bytes through its staging slot: each lane puts its row's four 16-byte units, then every
+// group of four lanes writes one row's 64 contiguous bytes (whole sectors; straight from the accumulator layout a
+// store would touch 32 rows with 16 bytes each). Unit u of row r lies at u ^ ((r / 2) & 3): conflict-free both ways.
+__device__ __forceinline__ void store_rows(uint4* slot, int lane, const uint4 (&unit)[4], char* out, int64_t row_bytes) {
+    __syncwarp();   // the previous rows' reads
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ex[e] = g.extra[(int64_t)row * 4 + e];
+    for (int u = 0; u < 4; ++u) slot[lane * 4 + (u ^ ((lane >> 1) & 3))] = unit[u];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int r = k * 8 + (lane >> 2), u = lane & 3;
+        *reinterpret_cast<uint4*>(out + r * row_bytes + 16 * u) = slot[r * 4 + (u ^ ((r >> 1) & 3))];
     }
-    for (int c0 = 0; c0 < COLS; c0 += 16) {
-        float v[16];
-        umma::tmem_ld16(trow + c0, v);
-        const int col = n0 + c0;
-        if (EPI == EPI_F32) {
-            float4* o = reinterpret_cast<float4*>(g.out_f32 + (int64_t)row * g.ldo + col);
+}
+
+// Fused epilogue of COLS accumulator columns of the warp's 32 rows (first row row0, the lane's row row0 + lane):
+// reads its TMEM lane starting at TMEM address `trow`, writes output columns n0 .. n0 + COLS - 1. The FP32 and
+// BF16 row-major outputs go through the warp's staging slot; the training path's other outputs (pre-activations,
+// transposed copies) are written directly.
+template <int COLS, int EPI>
+__device__ __forceinline__ void epilogue_cols(const GemmArgs& g, uint4* slot, uint32_t trow, int row0, int lane, int n0) {
+    const int row = row0 + lane;
+    if constexpr (EPI == EPI_F32 || EPI == EPI_BIAS) {
+        for (int c0 = 0; c0 < COLS; c0 += 16) {
+            float v[16];
+            umma::tmem_ld16(trow + c0, v);
+            const int col = n0 + c0;
+            if (EPI == EPI_BIAS) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else if (EPI == EPI_BIAS) {
-            float4* o = reinterpret_cast<float4*>(g.out_f32 + (int64_t)row * g.ldo + col);
+                for (int i = 0; i < 16; ++i) v[i] += __ldg(g.bias + col + i);
+                if (g.clamp_lo) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] += g.bias[col + i];
-            if (g.clamp_lo) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = fminf(fmaxf(v[i], g.clamp_lo[col + i]), g.clamp_hi[col + i]);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        } else {
-            __nv_bfloat16 h[16];
-            float u[16];
-            if (EPI == EPI_BIAS_GELU) {
-                const float4* bp = reinterpret_cast<const float4*>(g.bias + col);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 bb = __ldg(bp + i);
-                    u[4 * i] = bb.x; u[4 * i + 1] = bb.y; u[4 * i + 2] = bb.z; u[4 * i + 3] = bb.w;
-                }
-            } else {
-                const float4* pp = reinterpret_cast<const float4*>(g.pre + (int64_t)row * g.ldp + col);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 q = pp[i];
-                    u[4 * i] = q.x; u[4 * i + 1] = q.y; u[4 * i + 2] = q.z; u[4 * i + 3] = q.w;
+                    for (int i = 0; i < 16; ++i) v[i] = fminf(fmaxf(v[i], g.clamp_lo[col + i]), g.clamp_hi[col + i]);
                 }
             }
+            uint4 unit[4];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float z = v[i];
+            for (int u = 0; u < 4; ++u)
+                unit[u] = make_uint4(__float_as_uint(v[4 * u]), __float_as_uint(v[4 * u + 1]), __float_as_uint(v[4 * u + 2]),
+                                     __float_as_uint(v[4 * u + 3]));
+            store_rows(slot, lane, unit, reinterpret_cast<char*>(g.out_f32 + (int64_t)row0 * g.ldo + col), g.ldo * 4);
+        }
+    } else {
+        float ex[4] = {0.f, 0.f, 0.f, 0.f};
+        if (EPI == EPI_BIAS_GELU && g.extra) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ex[e] = g.extra[(int64_t)row * 4 + e];
+        }
+        for (int c0 = 0; c0 < COLS; c0 += 32) {
+            __align__(16) __nv_bfloat16 h[32];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float v[16];
+                umma::tmem_ld16(trow + c0 + 16 * half, v);
+                const int col = n0 + c0 + 16 * half;
+                float u[16];
                 if (EPI == EPI_BIAS_GELU) {
-                    z += u[i];
-                    if (g.wextra) {
-                        const float4 we = __ldg(reinterpret_cast<const float4*>(g.wextra) + col + i);
-                        z = fmaf(ex[0], we.x, fmaf(ex[1], we.y, fmaf(ex[2], we.z, fmaf(ex[3], we.w, z))));
+                    const float4* bp = reinterpret_cast<const float4*>(g.bias + col);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 bb = __ldg(bp + i);
+                        u[4 * i] = bb.x; u[4 * i + 1] = bb.y; u[4 * i + 2] = bb.z; u[4 * i + 3] = bb.w;
                     }
-                    if (g.out_f32) g.out_f32[(int64_t)row * g.ldo + col + i] = z;
-                    z = gelu(z);
-                } else {  // EPI_GELU_BWD: upstream gradient times GELU'(pre-activation)
-                    z *= gelu_grad(u[i]);
+                } else {
+                    const float4* pp = reinterpret_cast<const float4*>(g.pre + (int64_t)row * g.ldp + col);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 q = pp[i];
+                        u[4 * i] = q.x; u[4 * i + 1] = q.y; u[4 * i + 2] = q.z; u[4 * i + 3] = q.w;
+                    }
                 }
-                h[i] = __float2bfloat16_rn(z);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float z = v[i];
+                    if (EPI == EPI_BIAS_GELU) {
+                        z += u[i];
+                        if (g.wextra) {
+                            const float4 we = __ldg(reinterpret_cast<const float4*>(g.wextra) + col + i);
+                            z = fmaf(ex[0], we.x, fmaf(ex[1], we.y, fmaf(ex[2], we.z, fmaf(ex[3], we.w, z))));
+                        }
+                        if (g.out_f32) g.out_f32[(int64_t)row * g.ldo + col + i] = z;
+                        z = gelu(z);
+                    } else {  // EPI_GELU_BWD: upstream gradient times GELU'(pre-activation)
+                        z *= gelu_grad(u[i]);
+                    }
+                    h[16 * half + i] = __float2bfloat16_rn(z);
+                }
+                if (g.out_bf16_t) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) g.out_bf16_t[(int64_t)(col + i) * g.ldt + row] = h[16 * half + i];
+                }
             }
             if (g.out_bf16) {
-                uint4* o = reinterpret_cast<uint4*>(g.out_bf16 + (int64_t)row * g.ldh + col);
-                o[0] = *reinterpret_cast<const uint4*>(&h[0]);
-                o[1] = *reinterpret_cast<const uint4*>(&h[8]);
-            }
-            if (g.out_bf16_t) {
+                uint4 unit[4];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) g.out_bf16_t[(int64_t)(col + i) * g.ldt + row] = h[i];
+                for (int k = 0; k < 4; ++k) unit[k] = *reinterpret_cast<const uint4*>(&h[8 * k]);
+                store_rows(slot, lane, unit, reinterpret_cast<char*>(g.out_bf16 + (int64_t)row0 * g.ldh + n0 + c0), g.ldh * 2);
             }
         }
     }
@@ -250,6 +279,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     } else {
         // ---- epilogue (warps 2-17: TMEM lane quadrant warp % 4, column quarter (warp - 2) / 4) ----
         const int quad = warp & 3, part = (warp - EPI_WARP0) >> 2;
+        uint4* slot = reinterpret_cast<uint4*>(smem_raw + (base - umma::smem_u32(smem_raw)) + STAGES * S::STAGE) +
+                      (warp - EPI_WARP0) * 128;
         int local = 0;
         for (int t = blockIdx.x; t < tiles && !*abort_flag; t += gridDim.x, ++local) {
             const int b = local & 1;
@@ -257,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             umma::fence_after_sync();
             const int m0 = (t / tiles_n) * BM, n0 = (t % tiles_n) * BN;
             const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN + part * (BN / 4));
-            epilogue_cols<BN / 4, EPI>(g, trow, m0 + quad * 32 + lane, n0 + part * (BN / 4));
+            epilogue_cols<BN / 4, EPI>(g, slot, trow, m0 + quad * 32, lane, n0 + part * (BN / 4));
             umma::fence_before_sync();
             mbar_arrive(umma::smem_u32(&acc_empty[b]));
         }
