@@ -56,10 +56,14 @@ enum { PASS = 0, PASS_CURRENTS = 1, STAGE = 2, STAGE_RATES = 3 };
 // row but spills at 128 registers (two CTAs per SM) and was slower, 1.29 against 0.99 ms per stage at
 // 448 x 448 x 32 x 36 (1.17 at 168 registers, 12 warps per SM).
 template <bool AL, int ROWV, int XM, int YM, int MODE>
-__device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, int* sg, int n, int tx, int js,
-                                              int je) {
+__device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, Q* priv, int* sg, int n,
+                                              int tx, int js, int je) {
     using LV = LaneVec<float>;
     constexpr bool MIXED = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
+    // whole vectors, no currents: rows and c_g by cp.async (874 against 966 us per stage with the SourceTermSet
+    // rates at 384 x 384 x 32 x 36, 704 against 734 without at 601 x 417 x 24 x 24; with currents 1040 against 996
+    // at 448 x 448, element by element 542 against 418)
+    constexpr bool ASYNC = AL && !curr;
     static_assert(MIXED == (YM == MIX), "uniform in both directions or general");
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, L = p.L, CX = p.CX;
     const int64_t slice = (int64_t)Nx * Ny * Nk;
@@ -99,10 +103,36 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
     }
     if (hal)
         for (int d = 0; d <= 2; ++d) put(d + 3, hal_off, ld(modr(js + d), hcol));
-    Q nw = ld(modr(js + 3), colm), hv = hal ? ld(modr(js + 3), hcol) : qz();
+    // row j+3 comes one row ahead: by cp.async straight into the ring and c_g into a slot of the thread (ASYNC),
+    // or through registers
+    Q nw = qz(), hv = qz();
     Q vx = qz(), vy = qz(), vc = {f2(1.f), f2(1.f)};
+    Q* mine = priv + tid;
+    auto rload = [&](int s, int r) {
+        if constexpr (ASYNC) {
+            const float* src = base + r * rs + colm;
+            if (act) {
+                copy_async<AL>(ring + s * ROWV + own_off, src, left);
+                copy_async<AL>(ring + (s + 8) * ROWV + own_off, src, left);
+            }
+            if (hal) {
+                const float* hsrc = base + r * rs + hcol;
+                copy_async<AL>(ring + s * ROWV + hal_off, hsrc, left);
+                copy_async<AL>(ring + (s + 8) * ROWV + hal_off, hsrc, left);
+            }
+        } else {
+            nw = ld(r, colm);
+            if (hal) hv = ld(r, hcol);
+        }
+    };
+    rload(6, modr(js + 3));
     auto vload = [&](int r) {
         const int e = r * rs + colm;
+        if constexpr (ASYNC) {
+            if (cgp) copy_async<AL>(mine, p.cg + e, left);
+            copy_commit();
+            return;
+        }
         if (curr) {
             vx = ldgv<AL>(p.ux + e, left);
             vy = ldgv<AL>(p.uy + e, left);
@@ -113,6 +143,9 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
     auto velo = [&](Q& ux, Q& uy) {
         ux = gx;
         uy = gy;
+        if constexpr (ASYNC) copy_wait<0>();
+        if constexpr (ASYNC)
+            if (cgp) vc = lds(mine);
         if (cgp) {
             ux = qmul(vc, ux);
             uy = qmul(vc, uy);
@@ -161,16 +194,25 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
         const bool row = k < cnt;
         Q ux1 = qz();
         if (row) {
-            if (act) put(sw, own_off, nw);
-            if (hal) put(sw, hal_off, hv);
+            if constexpr (!ASYNC) {
+                if (act) put(sw, own_off, nw);
+                if (hal) put(sw, hal_off, hv);
+            }
             if constexpr (MIXED)
                 if (act) sg[(buf * (CX + 1) + slot) * L + l] = own ? codeq(ux0) : 0;
-            velo(ux1, uy1);
-            nw = ld(rl, colm);
-            if (hal) hv = ld(rl, hcol);
-            vload(rv);
+            velo(ux1, uy1);   // also waits for row j+3
+            if constexpr (!ASYNC) {
+                rload(0, rl);
+                vload(rv);
+            }
         }
         __syncthreads();
+        if constexpr (ASYNC) {
+            if (row) {   // row j+4 into the slot of row j-4, whose readers have passed a barrier since
+                rload((sw + 1) & 7, rl);
+                vload(rv);
+            }
+        }
         // the previous row: its lower x face from the left neighbour's candidates, then S
         if (k > 0 && slot >= 1) {
             Q Flo;
@@ -533,7 +575,7 @@ __device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* sm
     if constexpr (std::is_same<T, float>::value) {
         constexpr int ROWV = XTHREADS + 5 * LB;
         Q* ring = reinterpret_cast<Q*>(smem);
-        xyw_body_ring<AL, ROWV, XM, YM, MODE>(p, ring, ring + 16 * ROWV, sg, n, tx, js, je);
+        xyw_body_ring<AL, ROWV, XM, YM, MODE>(p, ring, ring + 16 * ROWV, ring + 16 * ROWV + 4 * XTHREADS, sg, n, tx, js, je);
     } else {
         D* rows = reinterpret_cast<D*>(smem);
         xyw_body<AL, XM, YM, MODE>(p, rows, rows + 2 * ROWV64, rows + 2 * ROWV64 + 4 * XTHREADS, sg, n, tx, js, je);
@@ -543,7 +585,8 @@ __device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* sm
 // Shared memory: the staged rows, then the x faces of two rows (two candidates each in the general body), FP64
 // then the threads' private slots.
 template <typename T, int LB> constexpr size_t xyw_smem() {
-    return ((std::is_same<T, float>::value ? 16 * (XTHREADS + 5 * LB) : 2 * ROWV64 + 5 * XTHREADS) + 4 * XTHREADS) * 16;
+    return ((std::is_same<T, float>::value ? 16 * (XTHREADS + 5 * LB) + (LB <= 8 ? 1 : 0) * XTHREADS : 2 * ROWV64 + 5 * XTHREADS) +
+            4 * XTHREADS) * 16;
 }
 
 // One CTA per (direction, x tile, row segment), direction fastest so the CTAs of one region run together.
