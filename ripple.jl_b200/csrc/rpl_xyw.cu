@@ -23,7 +23,7 @@ using namespace xyw;
 // (c the per-cell c_g magnitude, or 1 when c_g is folded into the direction table), enlarged by 1e-5,
 // at rmax[(2 region + axis) Nk + m] as bit patterns (non-negative floats order like them). One thread per
 // (bin, column, VROWS rows of a segment).
-constexpr int VROWS = 8;
+constexpr int VROWS = 4;
 
 template <typename T>
 __global__ void vel_kernel(int Nx, int Ny, int Nk, int per_tile, int tiles_x, int seg_rows, const double* __restrict__ coef,
@@ -77,7 +77,7 @@ bool walk_supported(const rpl_desc& d) {
 // Cells per CTA: as many as 256 threads hold, spread evenly over the tiles a row needs (a row of 64 cells
 // takes one tile of 65 slots, not one of 128 with half of them idle). Rows per segment: a segment pays a
 // prologue of six row loads and one face per column, so long segments are cheaper, but a small grid then
-// leaves SMs without a CTA: the largest of 128, 64, 32, 16, 8 rows that still gives three CTAs per SM.
+// leaves SMs without a CTA: the largest of 128, 64, 32, 16, 8, 4 rows that gives two CTAs per SM.
 WalkGeom walk_geometry(const rpl_desc& d) {
     WalkGeom g;
     const int N = d.precision == RPL_FP64 ? 2 : 4;
@@ -87,7 +87,7 @@ WalkGeom walk_geometry(const rpl_desc& d) {
     g.CX = (int)((d.Nx + g.tiles_x - 1) / g.tiles_x) + 1;
     g.threads = ((std::max(g.CX, 5) * g.L + 31) / 32) * 32;   // at least the five halo columns' threads
     g.seg = 128;
-    while (g.seg > 8 && d.Np * g.tiles_x * ((d.Ny + g.seg - 1) / g.seg) < 3 * 148) g.seg /= 2;
+    while (g.seg > 4 && d.Np * g.tiles_x * ((d.Ny + g.seg - 1) / g.seg) < 2 * 148) g.seg /= 2;
     return g;
 }
 
