@@ -855,9 +855,7 @@ int rpl_smooth_rows_async(rpl_handle* hh, double dt, int64_t row0, int64_t nrows
 int rpl_sync(rpl_handle* hh) {
     int st = check_handle(hh);
     if (st) return st;
-    Handle* h = reinterpret_cast<Handle*>(hh);
-    RPL_CUDA(cudaStreamSynchronize(h->stream));
-    return check_error_word(h);
+    return check_error_word(reinterpret_cast<Handle*>(hh));   // drains the stream
 }
 
 int rpl_set_stream(rpl_handle* hh, void* stream) {

@@ -165,11 +165,11 @@ __global__ void __launch_bounds__(256) terms_kernel(const T* __restrict__ N, Ter
 // per-cell values (x0, x1), written to tcol[c * n + t]. terms_bins_kernel: the rates of every bin from them.
 //
 // terms_cols_kernel: columns by lane vectors (rpl_colvec.cuh), the tables (weights and the three of the first
-// mean-spectrum term) in shared memory. One column per warp with the tables read through L1 took 822 us at
+// mean-spectrum term) in shared memory, an entry serving two columns per lane. One column per warp with the tables read through L1 took 822 us at
 // 384 x 384 x 32 x 36; reading the action once is 105 us.
 template <typename T, bool AL, bool SMEM>
 __global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict__ N, TermsArgs a, double2* __restrict__ tcol) {
-    constexpr int VN = ColVec<T>::N, CH = 12;
+    constexpr int VN = ColVec<T>::N, CH = 6;
     extern __shared__ __align__(16) double s_tab[];   // weights, then the three tables of the mean-spectrum term
     const int Nk = (int)a.Nk, Np = (int)a.Np, nb = Nk * Np, stride = table_stride<T>(Nk), size = stride * Np;
     int tm = -1;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict_
         __syncthreads();
     }
     const ColVec<T> v(Nk);
-    const int64_t slice = a.P * Nk, groups = (a.P + v.cpw - 1) / v.cpw;
+    const int64_t slice = a.P * Nk, groups = (a.P + 2 * v.cpw - 1) / (2 * v.cpw);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     // sum over the column's lanes, complete in its first lane
     auto fold = [&](double x) {
@@ -195,17 +195,22 @@ __global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict_
         return x;
     };
     for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
-        const int64_t col = g * v.cpw + v.col(), c = min(col, a.P - 1);
-        // two partial sums each (even and odd directions)
-        double m0p[2] = {}, skp[2] = {}, ssp[2] = {}, sdp[2] = {};
+        const int64_t col0 = g * 2 * v.cpw + v.col();   // this lane's columns: col0 and col0 + cpw
+        const int64_t cs[2] = {min(col0, a.P - 1), min(col0 + v.cpw, a.P - 1)};
+        double sums[2][4] = {};   // m0, then the integrals of N > 0 with k^p, sigma^p and 1
         for (int mm = v.l * VN; mm < Nk; mm += 32 * VN) {
-            const T* p = N + c * Nk + mm;
+            const T* p[2] = {N + cs[0] * Nk + mm, N + cs[1] * Nk + mm};
             const int left = Nk - 1 - mm;
-            for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
-                T f[CH][VN];
+            for (int n0 = 0; n0 < Np; n0 += CH) {
+                T f[CH][2][VN];
 #pragma unroll
-                for (int k = 0; k < CH; ++k)
-                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, f[k]);
+                for (int k = 0; k < CH; ++k) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        if (n0 + k < Np) ld_bins<AL>(p[j], left, f[k][j]);
+                        p[j] += slice;
+                    }
+                }
 #pragma unroll
                 for (int k = 0; k < CH; ++k) {
                     if (n0 + k >= Np) break;
@@ -213,66 +218,78 @@ __global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict_
                     for (int q = 0; q < VN; ++q) {
                         const int at = (n0 + k) * stride + mm + q, gb = (n0 + k) * Nk + mm + min(q, left);
                         const double in = SMEM || q <= left ? 1.0 : 0.0;
-                        const double x = (double)f[k][q];
-                        m0p[k & 1] = fma(x, SMEM ? s_tab[at] : in * __ldg(a.weights + gb), m0p[k & 1]);
+                        const double w = SMEM ? s_tab[at] : in * __ldg(a.weights + gb);
+                        double tk = 0.0, ts = 0.0, td = 0.0;
                         if (tm >= 0) {
-                            const double xp = f[k][q] > T(0) ? x : 0.0;
-                            skp[k & 1] = fma(xp, SMEM ? s_tab[size + at] : in * __ldg(tbm + gb), skp[k & 1]);
-                            ssp[k & 1] = fma(xp, SMEM ? s_tab[2 * size + at] : in * __ldg(tbm + nb + gb), ssp[k & 1]);
-                            sdp[k & 1] = fma(xp, SMEM ? s_tab[3 * size + at] : in * __ldg(tbm + 2 * nb + gb), sdp[k & 1]);
+                            tk = SMEM ? s_tab[size + at] : in * __ldg(tbm + gb);
+                            ts = SMEM ? s_tab[2 * size + at] : in * __ldg(tbm + nb + gb);
+                            td = SMEM ? s_tab[3 * size + at] : in * __ldg(tbm + 2 * nb + gb);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const double x = (double)f[k][j][q], xp = f[k][j][q] > T(0) ? x : 0.0;
+                            sums[j][0] = fma(x, w, sums[j][0]);
+                            if (tm >= 0) {
+                                sums[j][1] = fma(xp, tk, sums[j][1]);
+                                sums[j][2] = fma(xp, ts, sums[j][2]);
+                                sums[j][3] = fma(xp, td, sums[j][3]);
+                            }
                         }
                     }
                 }
             }
         }
-        const double m0 = fold(m0p[0] + m0p[1]);
-        const double sk = fold(skp[0] + skp[1]), ss = fold(ssp[0] + ssp[1]), sd = fold(sdp[0] + sdp[1]);
-        for (int t = 0; t < a.n; ++t) {
-            double msk = sk, mss = ss, msd = sd;
-            if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM && t != tm) {   // a further mean-spectrum term: its own pass
-                const double* tb = a.tabs + (int64_t)t * TABS * nb;
-                double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-                for (int n = 0; n < Np; ++n)
-                    for (int m = v.l; m < Nk; m += v.L) {
-                        const double x = (double)N[slice * n + c * Nk + m];
-                        const int b = m + Nk * n;
-                        if (x > 0.0) {
-                            f0 += x * tb[nb + b];
-                            f1 += x * tb[2 * nb + b];
-                            f2 += x * tb[3 * nb + b];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int64_t col = col0 + j * v.cpw, c = cs[j];
+            const double m0 = fold(sums[j][0]), sk = fold(sums[j][1]), ss = fold(sums[j][2]), sd = fold(sums[j][3]);
+            for (int t = 0; t < a.n; ++t) {
+                double msk = sk, mss = ss, msd = sd;
+                if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM && t != tm) {   // a further mean-spectrum term: its own pass
+                    const double* tb = a.tabs + (int64_t)t * TABS * nb;
+                    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+                    for (int n = 0; n < Np; ++n)
+                        for (int m = v.l; m < Nk; m += v.L) {
+                            const double x = (double)N[slice * n + c * Nk + m];
+                            const int b = m + Nk * n;
+                            if (x > 0.0) {
+                                f0 += x * tb[nb + b];
+                                f1 += x * tb[2 * nb + b];
+                                f2 += x * tb[3 * nb + b];
+                            }
                         }
-                    }
-                msk = fold(f0);
-                mss = fold(f1);
-                msd = fold(f2);
-            }
-            if (v.l != 0 || !v.used || col >= a.P) continue;
-            const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
-            double x0 = 0.0, x1 = 0.0;
-            switch (a.kind[t]) {
-                case RPL_TERM_EXPONENTIAL_WIND:
-                    x0 = rate;
-                    break;
-                case RPL_TERM_WAVE_AGE_WIND:
-                    x0 = rate;
-                    x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
-                    break;
-                case RPL_TERM_WHITECAPPING:
-                    x0 = rate * pow_nonneg(fmax(m0 / a.p[t][0] - 1.0, 0.0), a.p[t][1]);
-                    break;
-                default: {  // mean spectrum: the rate of bin k is x0 k + x1 k^2 (both 0: no dissipation)
-                    const double q = a.p[t][3];
-                    const double kbar = msd > 0.0 ? pow(msk / msd, 1.0 / q) : 0.0;
-                    const double sbar = msd > 0.0 ? pow(mss / msd, 1.0 / q) : 0.0;
-                    if (m0 > 0.0 && kbar > 0.0) {
-                        const double alpha = m0 * kbar * kbar, cs = -a.p[t][0] * alpha * alpha * sbar;
-                        x0 = cs * a.p[t][1] / kbar;
-                        x1 = cs * a.p[t][2] / (kbar * kbar);
-                    }
-                    break;
+                    msk = fold(f0);
+                    mss = fold(f1);
+                    msd = fold(f2);
                 }
+                if (v.l != 0 || !v.used || col >= a.P) continue;
+                const double rate = a.rate_field[t] ? a.rate_field[t][c] : a.rate[t];
+                double x0 = 0.0, x1 = 0.0;
+                switch (a.kind[t]) {
+                    case RPL_TERM_EXPONENTIAL_WIND:
+                        x0 = rate;
+                        break;
+                    case RPL_TERM_WAVE_AGE_WIND:
+                        x0 = rate;
+                        x1 = a.speed_field[t] ? a.speed_field[t][c] : a.speed[t];
+                        break;
+                    case RPL_TERM_WHITECAPPING:
+                        x0 = rate * pow_nonneg(fmax(m0 / a.p[t][0] - 1.0, 0.0), a.p[t][1]);
+                        break;
+                    default: {  // mean spectrum: the rate of bin k is x0 k + x1 k^2 (both 0: no dissipation)
+                        const double q = a.p[t][3];
+                        const double kbar = msd > 0.0 ? pow(msk / msd, 1.0 / q) : 0.0;
+                        const double sbar = msd > 0.0 ? pow(mss / msd, 1.0 / q) : 0.0;
+                        if (m0 > 0.0 && kbar > 0.0) {
+                            const double alpha = m0 * kbar * kbar, cd = -a.p[t][0] * alpha * alpha * sbar;
+                            x0 = cd * a.p[t][1] / kbar;
+                            x1 = cd * a.p[t][2] / (kbar * kbar);
+                        }
+                        break;
+                    }
+                }
+                tcol[c * a.n + t] = make_double2(x0, x1);
             }
-            tcol[c * a.n + t] = make_double2(x0, x1);
         }
     }
 }
@@ -284,58 +301,109 @@ __global__ void __launch_bounds__(256, 2) terms_cols_kernel(const T* __restrict_
 // 384 x 384 x 32 x 36; writing the rates once is 105 us).
 constexpr int TERM_COLS = 128;   // columns per thread in terms_bins_kernel (more on very large grids)
 
-// LINEAR_POWER: every wave-age term has power 1 (the reference's default); else pow_nonneg.
-template <typename T, int NT, bool LINEAR_POWER>
-__global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, const double2* __restrict__ tcol, T* __restrict__ R,
-                                                         int64_t chunk) {
+// The last NW of the NT terms are wave-age inputs (order[] lists the terms so), so that the loop over columns is
+// straight-line code and several columns' chains overlap. LINEAR_POWER: every wave-age term has power 1 (the
+// reference's default); else pow_nonneg.
+template <typename T, int NT, int NW, bool LINEAR_POWER>
+__global__ void __launch_bounds__(256) terms_bins_kernel(TermsArgs a, int4 order, const double2* __restrict__ tcol,
+                                                         T* __restrict__ R, int64_t chunk) {
     __shared__ double2 s_col[TERM_COLS * NT];
     const int64_t nb = a.Nk * a.Np;
     const int64_t bin = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, b = min(bin, nb - 1);
     const int64_t Nk = a.Nk, m = b % Nk, n = b / Nk;
     const int64_t c0 = (int64_t)blockIdx.y * chunk, c1 = min(c0 + chunk, a.P);
-    double A[NT], B[NT];
-    bool wave_age[NT];
+    const int id[4] = {order.x, order.y, order.z, order.w};
+    double A[NT], B[NT], threshold[NT], power[NT];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
+    for (int k = 0; k < NT; ++k) {
+        const int t = id[k];
         const double* tb = a.tabs + (int64_t)t * TABS * nb;
         const double t0 = tb[b];
-        A[t] = t0;
-        B[t] = 0.0;
-        wave_age[t] = a.kind[t] == RPL_TERM_WAVE_AGE_WIND;
-        if (wave_age[t]) {
+        A[k] = t0;
+        B[k] = 0.0;
+        threshold[k] = power[k] = 0.0;
+        if (k >= NT - NW) {
             // x0 B max(x1 A - threshold, 0)^power, A = alignment / phase speed; a bin off the wind has no growth
             // whatever the powers (0^0 = 1): B = 0 there
-            A[t] = t0 * tb[nb + b];
-            B[t] = t0 > 0.0 ? tb[2 * nb + b] : 0.0;
+            A[k] = t0 * tb[nb + b];
+            B[k] = t0 > 0.0 ? tb[2 * nb + b] : 0.0;
+            threshold[k] = a.p[t][0];
+            power[k] = a.p[t][1];
         } else if (a.kind[t] == RPL_TERM_WHITECAPPING) {
-            A[t] = -t0;
+            A[k] = -t0;
         } else if (a.kind[t] == RPL_TERM_MEAN_SPECTRUM) {
-            A[t] = -t0;
-            B[t] = -t0 * t0;
+            A[k] = -t0;
+            B[k] = -t0 * t0;
         }
     }
     T* out = R + n * a.P * Nk + m;
     for (int64_t s0 = c0; s0 < c1; s0 += TERM_COLS) {
         const int cols = (int)min((int64_t)TERM_COLS, c1 - s0);
         __syncthreads();
-        for (int k = threadIdx.x; k < cols * NT; k += 256) s_col[k] = tcol[s0 * NT + k];
+        for (int k = threadIdx.x; k < cols * NT; k += 256) {
+            const int c = k / NT, t = k - c * NT;
+            s_col[k] = tcol[(s0 + c) * NT + (t == 0 ? id[0] : (t == 1 ? id[1] : (t == 2 ? id[2] : id[3])))];
+        }
         __syncthreads();
         if (bin >= nb) continue;
+        T* at = out + s0 * Nk;
 #pragma unroll 4
-        for (int k = 0; k < cols; ++k) {
-            double r = 0.0;
+        for (int k = 0; k < cols; ++k, at += Nk) {
+            double lin = 0.0, win = 0.0;
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 const double2 x = s_col[k * NT + t];
-                if (!wave_age[t]) {
-                    r = fma(x.x, A[t], fma(x.y, B[t], r));
+                if (t < NT - NW) {
+                    lin = fma(x.x, A[t], lin);
+                    win = fma(x.y, B[t], win);
                 } else {
-                    const double excess = fmax(fma(x.y, A[t], -a.p[t][0]), 0.0);
-                    r = fma(x.x * B[t], LINEAR_POWER ? excess : pow_nonneg(excess, a.p[t][1]), r);
+                    const double e = fma(x.y, A[t], -threshold[t]), excess = e > 0.0 ? e : 0.0;
+                    win = fma(x.x * B[t], LINEAR_POWER ? excess : pow_nonneg(excess, power[t]), win);
                 }
             }
-            out[(s0 + k) * Nk] = (T)r;
+            *at = (T)(lin + win);
         }
+    }
+}
+
+template <typename T, int NT, int NW>
+cudaError_t bins_nw(const TermsArgs& a, int4 order, bool linear, const double2* tcol, T* R, int64_t chunk, dim3 grid, cudaStream_t s) {
+    if (linear) terms_bins_kernel<T, NT, NW, true><<<grid, 256, 0, s>>>(a, order, tcol, R, chunk);
+    else terms_bins_kernel<T, NT, NW, false><<<grid, 256, 0, s>>>(a, order, tcol, R, chunk);
+    return cudaGetLastError();
+}
+
+template <typename T, int NT>
+cudaError_t bins_nt(const TermsArgs& a, const double2* tcol, T* R, int64_t chunk, dim3 grid, cudaStream_t s) {
+    int id[4] = {0, 0, 0, 0}, k = 0, nw = 0;
+    bool linear = true;
+    for (int t = 0; t < NT; ++t)
+        if (a.kind[t] != RPL_TERM_WAVE_AGE_WIND) id[k++] = t;
+    for (int t = 0; t < NT; ++t)
+        if (a.kind[t] == RPL_TERM_WAVE_AGE_WIND) {
+            id[k++] = t;
+            ++nw;
+            linear = linear && a.p[t][1] == 1.0;
+        }
+    const int4 order = make_int4(id[0], id[1], id[2], id[3]);
+    if (nw == 0) return bins_nw<T, NT, 0>(a, order, true, tcol, R, chunk, grid, s);
+    if (nw == 1) return bins_nw<T, NT, 1>(a, order, linear, tcol, R, chunk, grid, s);
+    if constexpr (NT >= 2)
+        if (nw == 2) return bins_nw<T, NT, 2>(a, order, linear, tcol, R, chunk, grid, s);
+    if constexpr (NT >= 3)
+        if (nw == 3) return bins_nw<T, NT, 3>(a, order, linear, tcol, R, chunk, grid, s);
+    if constexpr (NT >= 4) return bins_nw<T, NT, 4>(a, order, linear, tcol, R, chunk, grid, s);
+    return cudaErrorInvalidValue;
+}
+
+template <typename T>
+cudaError_t launch_bins(const TermsArgs& a, const double2* tcol, T* R, int64_t chunk, dim3 grid, cudaStream_t s) {
+    switch (a.n) {
+        case 1: return bins_nt<T, 1>(a, tcol, R, chunk, grid, s);
+        case 2: return bins_nt<T, 2>(a, tcol, R, chunk, grid, s);
+        case 3: return bins_nt<T, 3>(a, tcol, R, chunk, grid, s);
+        case 4: return bins_nt<T, 4>(a, tcol, R, chunk, grid, s);
+        default: return cudaErrorInvalidValue;
     }
 }
 
@@ -447,7 +515,7 @@ cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s) {
                            : (a.Nk % VN == 0 ? terms_cols_kernel<T, true, true> : terms_cols_kernel<T, false, true>);
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
             if (e != cudaSuccess) return e;
-            const int64_t per = 8 * (32 / std::min<int64_t>((a.Nk + VN - 1) / VN, 32));
+            const int64_t per = 16 * (32 / std::min<int64_t>((a.Nk + VN - 1) / VN, 32));
             k<<<(unsigned)std::min<int64_t>((a.P + per - 1) / per, 148 * 2), 256, used, s>>>(in, a, h.d_tcol);
             return cudaGetLastError();
         };
@@ -455,27 +523,8 @@ cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         const int64_t chunk = std::max<int64_t>(TERM_COLS, (a.P + 65534) / 65535);   // grid.y <= 65535
         const dim3 grid((unsigned)((a.Nk * a.Np + 255) / 256), (unsigned)((a.P + chunk - 1) / chunk));
-        bool linear = true;
-        for (int t = 0; t < a.n; ++t) linear = linear && (a.kind[t] != RPL_TERM_WAVE_AGE_WIND || a.p[t][1] == 1.0);
-        switch (a.n) {
-#define RPL_BINS(NT)                                                                                           \
-    case NT:                                                                                                   \
-        if (fp64) {                                                                                            \
-            if (linear) terms_bins_kernel<double, NT, true><<<grid, 256, 0, s>>>(a, h.d_tcol, (double*)h.d_lin_rates, chunk); \
-            else terms_bins_kernel<double, NT, false><<<grid, 256, 0, s>>>(a, h.d_tcol, (double*)h.d_lin_rates, chunk);       \
-        } else {                                                                                               \
-            if (linear) terms_bins_kernel<float, NT, true><<<grid, 256, 0, s>>>(a, h.d_tcol, (float*)h.d_lin_rates, chunk);   \
-            else terms_bins_kernel<float, NT, false><<<grid, 256, 0, s>>>(a, h.d_tcol, (float*)h.d_lin_rates, chunk);         \
-        }                                                                                                      \
-        break;
-            RPL_BINS(1)
-            RPL_BINS(2)
-            RPL_BINS(3)
-            RPL_BINS(4)
-#undef RPL_BINS
-            default: return cudaErrorInvalidValue;
-        }
-        return cudaGetLastError();
+        return fp64 ? launch_bins(a, h.d_tcol, (double*)h.d_lin_rates, chunk, grid, s)
+                    : launch_bins(a, h.d_tcol, (float*)h.d_lin_rates, chunk, grid, s);
     }
     if (fp64)
         terms_kernel<double><<<blocks, 256, 0, s>>>((const double*)Nin, a, (double*)h.d_lin_rates);

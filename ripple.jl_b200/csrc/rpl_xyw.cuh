@@ -22,8 +22,8 @@
 //    magnitude when the depth varies, else 1 with c_g in the table g), so it has the sign of g(m,n)
 //    wherever |g(m,n)| > |U| / c. vel_kernel stores, per region of cells and kappa bin, the maximum of
 //    |U| / c enlarged by 1e-5 (FP32); a CTA whose every bin passes |g| (1 - 1e-5) > that maximum, with
-//    one sign, runs the uniform body, every other CTA the general body (both candidates where needed,
-//    per-element selects). The margins cover the FP32 roundings of the product, the division and the
+//    one sign, runs a body without selects along that axis; elsewhere both candidates are reconstructed where
+//    needed and selected per element. The margins cover the FP32 roundings of the product, the division and the
 //    test. Both bodies give the same face values bit for bit (a stencil read backwards changes the sign
 //    of its odd differences only, exactly), in FP32 those of the fused tile kernel.
 #pragma once
@@ -59,12 +59,11 @@ template <bool AL, int ROWV, int XM, int YM, int MODE>
 __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, Q* priv, int* sg, int n,
                                               int tx, int js, int je) {
     using LV = LaneVec<float>;
-    constexpr bool MIXED = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
+    constexpr bool XMIX = XM == MIX, YMIX = YM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
     // whole vectors, no currents: rows and c_g by cp.async (874 against 966 us per stage with the SourceTermSet
     // rates at 384 x 384 x 32 x 36, 704 against 734 without at 601 x 417 x 24 x 24; with currents 1040 against 996
     // at 448 x 448, element by element 542 against 418)
     constexpr bool ASYNC = AL && !curr;
-    static_assert(MIXED == (YM == MIX), "uniform in both directions or general");
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, L = p.L, CX = p.CX;
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const int tid = threadIdx.x, l = tid % L;
@@ -167,7 +166,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
     velo(ux0, uy0);
     Q uy1 = qz();
     vload(modr(js + 1));
-    if (MIXED && slot == 0 && act) {
+    if (XMIX && slot == 0 && act) {
         sg[CX * L + l] = 0;
         sg[(2 * CX + 1) * L + l] = 0;
     }
@@ -198,7 +197,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
                 if (act) put(sw, own_off, nw);
                 if (hal) put(sw, hal_off, hv);
             }
-            if constexpr (MIXED)
+            if constexpr (XMIX)
                 if (act) sg[(buf * (CX + 1) + slot) * L + l] = own ? codeq(ux0) : 0;
             velo(ux1, uy1);   // also waits for row j+3
             if constexpr (!ASYNC) {
@@ -216,7 +215,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
         // the previous row: its lower x face from the left neighbour's candidates, then S
         if (k > 0 && slot >= 1) {
             Q Flo;
-            if constexpr (MIXED) {
+            if constexpr (XMIX) {
                 const Q* f = fsm + (((1 - buf) * CX + slot - 1) * L + l) * 2;
                 Flo = selq(ux_prev, lds(f), lds(f + 1));
             } else {
@@ -314,8 +313,7 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
     using LV = LaneVec<T>;
     using V = typename LV::V;
     constexpr int ROWV = ROWV64;
-    constexpr bool MIXED = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
-    static_assert(MIXED == (YM == MIX), "uniform in both directions or general");
+    constexpr bool XMIX = XM == MIX, YMIX = YM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, L = p.L, CX = p.CX;
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const int tid = threadIdx.x, l = tid % L;
@@ -383,7 +381,11 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
     // squares aw (POS: e[q] = d[q] - d[q-1]; NEG: e[q] = d[q] - d[q+1]). General body: rows j-2 .. j+3 in w.
     V sw[4], dw[4], ew[4], aw[4], w[6];
     V pLy = LV::zero(), pRy = LV::zero();   // the candidates of the lower y face of the current row
-    if constexpr (MIXED) {
+    if (XMIX && slot == 0 && act) {
+        sg[CX * L + l] = 0;
+        sg[(2 * CX + 1) * L + l] = 0;
+    }
+    if constexpr (YMIX) {
 #pragma unroll
         for (int d = -2; d <= 3; ++d) w[d + 2] = ld(modr(js + d), colm);
         const V below = ld(modr(js - 3), colm);
@@ -391,10 +393,6 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
         if (__any_sync(FULL, need & 1)) pLy = qweno(below, w[0], w[1], w[2], w[3]);
         if (__any_sync(FULL, need & 2)) pRy = qweno(w[4], w[3], w[2], w[1], w[0]);
         rload(0, modr(js + 4));
-        if (slot == 0 && act) {
-            sg[CX * L + l] = 0;
-            sg[(2 * CX + 1) * L + l] = 0;
-        }
     } else if constexpr (YM == POS) {
         const V r0 = ld(modr(js - 3), colm), r1 = ld(modr(js - 2), colm), r2 = ld(modr(js - 1), colm);
         sw[0] = ld(js, colm);
@@ -431,12 +429,12 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
     }
     if (hal) copy_async<AL>(hal_at, base + js * rs + hcol, left);
     // general body: the velocity of row j+1 is known during row j
-    if constexpr (MIXED) vload(modr(js + 1));
+    if constexpr (YMIX) vload(modr(js + 1));
     copy_commit();
     copy_wait<0>();
     // rows the next loads touch
-    constexpr int AHEAD = MIXED ? 5 : (YM == POS ? 3 : 4);
-    int rl = modr(js + AHEAD), rv = modr(js + (MIXED ? 2 : 1)), rh = modr(js + 1);
+    constexpr int AHEAD = YMIX ? 5 : (YM == POS ? 3 : 4);
+    int rl = modr(js + AHEAD), rv = modr(js + (YMIX ? 2 : 1)), rh = modr(js + 1);
     const T dxi = p.dx_inv, dyi = p.dy_inv;
     V Fx_prev = LV::zero(), fy_prev = LV::zero(), ux_prev = LV::zero();
     int outoff = js * rs + colm;
@@ -444,14 +442,13 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
         const int buf = k & 1;
         const bool row = k < cnt;
         V c, ux1 = LV::zero(), uy1 = LV::zero();
-        if constexpr (MIXED) c = w[2];
+        if constexpr (YMIX) c = w[2];
         else c = sw[0];
         if (row) {
             if (act) sts(own_at + buf * ROWV, c);
-            if constexpr (MIXED) {
+            if constexpr (XMIX)
                 if (act) sg[(buf * (CX + 1) + slot) * L + l] = own ? codeq(ux0) : 0;
-                velo(ux1, uy1);
-            }
+            if constexpr (YMIX) velo(ux1, uy1);
         }
         __syncthreads();
         if (row) {   // row j is complete in rowb; the other buffer's last readers have passed this barrier
@@ -463,7 +460,7 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
         // the previous row: its lower x face from the left neighbour's candidates, then S
         if (k > 0 && slot >= 1) {
             V Flo;
-            if constexpr (MIXED) {
+            if constexpr (XMIX) {
                 const V* f = fsm + (((1 - buf) * CX + slot - 1) * L + l) * 2;
                 Flo = selq(ux_prev, lds(f), lds(f + 1));
             } else {
@@ -474,7 +471,7 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
                 if (own) stv<AL>(Sn + outoff - rs, qadd(fx, fy_prev), left);
             } else {
                 V cv;                                          // the finished row's action
-                if constexpr (MIXED) cv = w[1];
+                if constexpr (YMIX) cv = w[1];
                 else cv = sw[3];
                 V G = qneg(qadd(fx, fy_prev));
                 if (RATES) G = qfma(plr, cv, G);             // SourceTermSet rates of this stage
@@ -511,7 +508,7 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
         }
         {
             V Fhi, Flo;
-            if constexpr (MIXED) {
+            if constexpr (YMIX) {
                 const int need = own ? (codeq(uy0) | (k + 1 < cnt ? codeq(uy1) : 0)) : 0;
                 V Ly = LV::zero(), Ry = LV::zero();
                 if (__any_sync(FULL, need & 1)) Ly = qweno(w[0], w[1], w[2], w[3], w[4]);
@@ -539,7 +536,7 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
             }
             fy_prev = qmuls(qmul(uy0, qsub(Fhi, Flo)), dyi);
         }
-        if constexpr (MIXED) {
+        if constexpr (YMIX) {
 #pragma unroll
             for (int q = 0; q < 5; ++q) w[q] = w[q + 1];
             w[5] = lds(mine + buf * XTHREADS);
@@ -623,17 +620,22 @@ xyw_kernel(const WalkArgs<T> p, int seg0) {
     }
     const int allxp = __syncthreads_and(xp), allxn = __syncthreads_and(xn);
     const int allyp = __syncthreads_and(yp), allyn = __syncthreads_and(yn);
-    const int xm = allxp ? POS : (allxn ? NEG : MIX);
-    const int ym = allyp ? POS : (allyn ? NEG : MIX);
-    // the four sign-uniform bodies, else the general one
-    if (xm == MIX || ym == MIX) run_body<T, AL, LB, MIX, MIX, MODE>(p, smem, sg, n, tx, js, je);
-    else if (xm == POS) {
-        if (ym == POS) run_body<T, AL, LB, POS, POS, MODE>(p, smem, sg, n, tx, js, je);
-        else run_body<T, AL, LB, POS, NEG, MODE>(p, smem, sg, n, tx, js, je);
-    } else {
-        if (ym == POS) run_body<T, AL, LB, NEG, POS, MODE>(p, smem, sg, n, tx, js, je);
-        else run_body<T, AL, LB, NEG, NEG, MODE>(p, smem, sg, n, tx, js, je);
-    }
+    const int xm = allxp ? POS : (allxn ? NEG : MIX), ym = allyp ? POS : (allyn ? NEG : MIX);
+    // one body per pair of signs, mixed ones included: 5 to 17% of the directions run along an axis, where one
+    // component's sign depends on the current. Against the four uniform bodies and one general body: 407 against
+    // 431 us per stage at 389 x 251 x 25 x 24 FP32, 1041 against 1068 at 320 x 320 x 32 x 36 FP64.
+#define RPL_BODY(X, Y) \
+    if (xm == X && ym == Y) return run_body<T, AL, LB, X, Y, MODE>(p, smem, sg, n, tx, js, je)
+    RPL_BODY(POS, POS);
+    RPL_BODY(POS, NEG);
+    RPL_BODY(NEG, POS);
+    RPL_BODY(NEG, NEG);
+    RPL_BODY(POS, MIX);
+    RPL_BODY(NEG, MIX);
+    RPL_BODY(MIX, POS);
+    RPL_BODY(MIX, NEG);
+    RPL_BODY(MIX, MIX);
+#undef RPL_BODY
 }
 
 template <typename T, bool AL, int LB, int MODE>
