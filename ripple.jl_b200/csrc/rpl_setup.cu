@@ -280,14 +280,14 @@ __device__ __forceinline__ void tadd(double& s, double& c, double v) {
 
 // Per-(i,j) moments (moments.jl:33-37,100-123), columns by lane vectors (rpl_colvec.cuh): per lane, FP64 sums of
 // blocks of four products folded into compensated totals, then a fixed-order compensated fold over the column's
-// lanes (deterministic). The error stays within a few units in the last place of the sum of |terms|.
+// lanes (deterministic); a table entry serves two columns per lane. The error stays within a few units in the last place of the sum of |terms|.
 // ALL = false computes m0 alone (for the total action), with the same arithmetic for m0. One column per warp
 // with the tables read through L1 took 802 us at 448 x 448 x 32 x 36; reading the state once is 143 us and its
 // FP64 work (a conversion, four FMAs and two compensated adds' share per bin) 150 us.
 template <typename T, bool AL, bool ALL, bool SMEM>
 __global__ void __launch_bounds__(256, 2)
 diag_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const double* __restrict__ tabs, double* __restrict__ out) {
-    constexpr int VN = ColVec<T>::N, TAB = ALL ? 4 : 1, DIRS = 4 / VN, CH = 12;   // a block: DIRS directions of VN bins
+    constexpr int VN = ColVec<T>::N, TAB = ALL ? 4 : 1, DIRS = 4 / VN, CH = 6;   // a block: DIRS directions of VN bins
     extern __shared__ __align__(16) double s_tab[];
     const int stride = table_stride<T>(Nk), size = stride * Np, nb = Nk * Np;
     if constexpr (SMEM) {
@@ -296,24 +296,29 @@ diag_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const double* __
         __syncthreads();
     }
     const ColVec<T> v(Nk);
-    const int64_t slice = P * Nk, groups = (P + v.cpw - 1) / v.cpw;
+    const int64_t slice = P * Nk, groups = (P + 2 * v.cpw - 1) / (2 * v.cpw);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
-        const int64_t col = g * v.cpw + v.col(), c = min(col, P - 1);
-        double s[TAB] = {}, e[TAB] = {};
+        const int64_t col0 = g * 2 * v.cpw + v.col();   // this lane's columns: col0 and col0 + cpw
+        const int64_t cs[2] = {min(col0, P - 1), min(col0 + v.cpw, P - 1)};
+        double s[2][TAB] = {}, e[2][TAB] = {};
         for (int m0 = v.l * VN; m0 < Nk; m0 += 32 * VN) {
-            const T* p = N + c * Nk + m0;
+            const T* p[2] = {N + cs[0] * Nk + m0, N + cs[1] * Nk + m0};
             const int left = Nk - 1 - m0;
-            for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
-                T a[CH][VN];
+            for (int n0 = 0; n0 < Np; n0 += CH) {
+                T a[CH][2][VN];
 #pragma unroll
                 for (int k = 0; k < CH; ++k) {
-                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, a[k]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        if (n0 + k < Np) ld_bins<AL>(p[j], left, a[k][j]);
+                        p[j] += slice;
+                    }
                 }
 #pragma unroll
                 for (int k0 = 0; k0 < CH; k0 += DIRS) {
                     if (n0 + k0 >= Np) break;
-                    double b[TAB] = {};
+                    double b[2][TAB] = {};
 #pragma unroll
                     for (int k = k0; k < k0 + DIRS; ++k) {
                         if (n0 + k >= Np) break;
@@ -323,33 +328,40 @@ diag_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const double* __
                             for (int q = 0; q < VN; ++q) {
                                 const double w = SMEM ? s_tab[t * size + (n0 + k) * stride + m0 + q]
                                                       : (q <= left ? __ldg(tabs + t * nb + (n0 + k) * Nk + m0 + q) : 0.0);
-                                b[t] = fma((double)a[k][q], w, b[t]);
+#pragma unroll
+                                for (int j = 0; j < 2; ++j) b[j][t] = fma((double)a[k][j][q], w, b[j][t]);
                             }
                     }
 #pragma unroll
-                    for (int t = 0; t < TAB; ++t) tadd(s[t], e[t], b[t]);
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int t = 0; t < TAB; ++t) tadd(s[j][t], e[j][t], b[j][t]);
                 }
             }
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
+        for (int j = 0; j < 2; ++j) {
 #pragma unroll
-            for (int t = 0; t < TAB; ++t) {
-                const double so = __shfl_down_sync(0xffffffffu, s[t], off), eo = __shfl_down_sync(0xffffffffu, e[t], off);
-                if (v.l + off < v.L) {
-                    tadd(s[t], e[t], so);
-                    e[t] += eo;
+            for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+                for (int t = 0; t < TAB; ++t) {
+                    const double so = __shfl_down_sync(0xffffffffu, s[j][t], off), eo = __shfl_down_sync(0xffffffffu, e[j][t], off);
+                    if (v.l + off < v.L) {
+                        tadd(s[j][t], e[j][t], so);
+                        e[j][t] += eo;
+                    }
                 }
             }
-        }
-        if (v.l == 0 && v.used && col < P) {
-            const double m0 = s[0] + e[0];
-            out[c] = m0;
-            if constexpr (ALL) {
-                const double mx = s[1] + e[1], my = s[2] + e[2], mt = s[3] + e[3];
-                out[P + c] = 4.0 * sqrt(m0);
-                out[2 * P + c] = sqrt(m0 == 0.0 ? 0.0 : mt / m0);
-                out[3 * P + c] = atan2(my, mx);
+            const int64_t col = col0 + j * v.cpw;
+            if (v.l == 0 && v.used && col < P) {
+                const double m0 = s[j][0] + e[j][0];
+                out[col] = m0;
+                if constexpr (ALL) {
+                    const double mx = s[j][1] + e[j][1], my = s[j][2] + e[j][2], mt = s[j][3] + e[j][3];
+                    out[P + col] = 4.0 * sqrt(m0);
+                    out[2 * P + col] = sqrt(m0 == 0.0 ? 0.0 : mt / m0);
+                    out[3 * P + col] = atan2(my, mx);
+                }
             }
         }
     }
@@ -596,7 +608,7 @@ cudaError_t launch_diagnostics(const Handle& h, const void* Nin, cudaStream_t s,
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
         if (e != cudaSuccess) return e;
         const int64_t cpw = 32 / std::min<int64_t>((d.Nk + ColVec<T>::N - 1) / ColVec<T>::N, 32);
-        const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(8 * cpw)), 148 * 2);
+        const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(16 * cpw)), 148 * 2);
         k<<<blocks, 256, used, s>>>(in, P, (int)d.Nk, (int)d.Np, h.d_weights, h.d_diag);
         return cudaGetLastError();
     };

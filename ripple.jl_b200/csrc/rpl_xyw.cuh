@@ -59,7 +59,7 @@ template <bool AL, int ROWV, int XM, int YM, int MODE>
 __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, Q* priv, int* sg, int n,
                                               int tx, int js, int je) {
     using LV = LaneVec<float>;
-    constexpr bool XMIX = XM == MIX, YMIX = YM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
+    constexpr bool XMIX = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
     // whole vectors, no currents: rows and c_g by cp.async (874 against 966 us per stage with the SourceTermSet
     // rates at 384 x 384 x 32 x 36, 704 against 734 without at 601 x 417 x 24 x 24; with currents 1040 against 996
     // at 448 x 448, element by element 542 against 418)
