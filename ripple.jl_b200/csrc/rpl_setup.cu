@@ -63,7 +63,7 @@ __global__ void q_column_table_kernel(int64_t P, int64_t Nz, int64_t Nk, const d
 
 // U[i,j,m] = sum_k uL[i,j,k] * W_m[k] (doppler_velocity.jl:45-62; with derivative the dF/dkappa
 // weights of :64-82), sequential in k like the reference. One warp per (i,j) column, lanes over the
-// kappa rings (chunks of 32); u, v are warp-uniform loads; U is written in device order c*Nk + m
+// kappa rings (chunks of 32); U is written in device order c*Nk + m
 // (coalesced). The weights come from a shared (Nz, Nk)
 // table (W, col_stride 0), a per-column table (col_stride Nz*Nk), or are evaluated here (W null; each
 // face once). z faces are strictly increasing (checked by the caller).
@@ -85,12 +85,19 @@ __global__ void doppler_kernel(int64_t Nx, int64_t Ny, int64_t Nz, int64_t Nk,
         const int64_t mm = active ? m : Nk - 1;
         double ax = 0.0, ay = 0.0;
         if (W) {
+            // 32 levels of u and v at a time, one per lane, handed round by shuffle: read warp-uniform level by
+            // level they queued behind the weights' streaming loads in L1 (296 us at 448 x 448 x 32 levels x 32)
             const TW* w = W + col * col_stride + mm;
-#pragma unroll 4
-            for (int64_t k = 0; k < Nz; ++k) {
-                const double wk = (double)__ldg(w + k * Nk);
-                ax += __ldg(u + col + P * k) * wk;
-                ay += __ldg(v + col + P * k) * wk;
+            for (int64_t k0 = 0; k0 < Nz; k0 += 32) {
+                const int nz = (int)min((int64_t)32, Nz - k0);
+                const int64_t at = col + P * (k0 + min(lane, nz - 1));
+                const double ul = __ldg(u + at), vl = __ldg(v + at);
+#pragma unroll 8
+                for (int q = 0; q < nz; ++q) {
+                    const double wk = (double)__ldg(w + (k0 + q) * Nk);
+                    ax += __shfl_sync(0xffffffffu, ul, q) * wk;
+                    ay += __shfl_sync(0xffffffffu, vl, q) * wk;
+                }
             }
         } else {
             const double kap = kappa[mm];
