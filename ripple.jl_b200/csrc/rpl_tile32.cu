@@ -338,15 +338,14 @@ __device__ __forceinline__ void tile_body(const TileArgs& p, int tile, float* sm
     asm volatile("cp.async.wait_group 0;");
 }
 
-// Refraction stages of FP32 models run as two kernels with smaller register footprints than the fused
-// tile body, so more warps hide the latency of the WENO5 chains (measured on seamount 1024^2 x 32 x 36:
-// 12.9 ms per stage against 14.4 ms fused, bit-identical results):
-//   xy_kernel (pass A): the tile body's staging of the phi planes and its x and y fluxes; writes
-//     S = fx/dx + fy/dy per cell-bin (state layout);
-//   kp_kernel (pass B): one thread per (cell, kappa pair) walking the phi ring with its register window,
-//     the kappa stencil from the cell's other lanes (warp shuffles, the reference's clamped indices),
-//     the kappa and phi fluxes, sources and the stage update: G = -(((S + fk) + fp)), the fused kernel's
-//     order of additions.
+// Refraction stages run as two kernels with smaller register footprints than the fused tile body, so more
+// warps hide the latency of the WENO5 chains. The forms of this file, bit-identical to the lane-vector forms:
+//   xy_kernel (RPL_PASS_A=tiles, and handles without velocity planes): the tile body's staging
+//     of the phi planes and its x and y fluxes; writes S = fx/dx + fy/dy per cell-bin (state layout);
+//   kp_kernel (second pass with the bundle or learned sources): one thread per (cell, kappa pair) walking the
+//     phi ring with its register window, the kappa stencil from the cell's other lanes (warp shuffles, the
+//     reference's clamped indices), the kappa and phi fluxes, sources and the stage update:
+//     G = -(((S + fk) + fp)), the fused kernel's order of additions.
 template <int L, int TX, int TY>
 __device__ __forceinline__ void xy_body(const TileArgs& p, int tile, float* smem) {
     float* S = p.sxy;
@@ -728,9 +727,9 @@ cudaError_t launch_variant(const TileArgs& a, int tiles, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// Two-pass refraction stage: pass A (the y-walk, or staged tiles with RPL_PASS_A=tiles), then pass B: the
-// ring walk with four kappa bins per lane without the bundle or learned sources, else (or with
-// RPL_PASS_B=pairs) the pair kernel in 256-thread CTAs.
+// Two-pass refraction stage: the x/y pass (the y-walk; staged tiles with RPL_PASS_A=tiles or without velocity
+// planes), then the ring walk with four kappa bins per lane without the bundle or learned sources, else (or
+// with RPL_PASS_B=pairs) the pair kernel in 256-thread CTAs.
 template <int L, int SRC>
 cudaError_t launch_split(const Handle& h, const StageParams& p, const TileArgs& a, const WalkArgs<float>& w,
                          cudaStream_t s) {
