@@ -135,6 +135,7 @@ int check_error_word(Handle* h) {
         RPL_CUDA(cudaStreamSynchronize(h->stream));
         if (w & 2u) return fail(RPL_ERR_NONFINITE, "non-finite values in the action passed in");
         if (w & 4u) return fail(RPL_ERR_DEVICE, "a tensor-core GEMM of the learned source gave up waiting");
+        if (w & 8u) return fail(RPL_ERR_DEVICE, "a stage kernel gave up waiting for a row");
         return fail(RPL_ERR_DEVICE, "a stage kernel produced non-finite wave action (time step too large?)");
     }
     return RPL_OK;

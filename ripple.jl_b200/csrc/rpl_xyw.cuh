@@ -50,20 +50,49 @@ enum { PASS = 0, PASS_CURRENTS = 1, STAGE = 2, STAGE_RATES = 3 };
 
 // FP32: the y stencil from a ring of staged rows in shared memory (16 rows of ROWV vectors; a row is written
 // twice, slots s and s+8, so the seven rows around j sit at constant offsets from one slot; row j+3 is
-// written before the step's barrier into the slot of row j-5, which no thread reads after the previous
-// barrier). The FP32 body is bound by the reciprocals (MUFU) and by how many warps hide them: holding the
+// written in step j into the slot of row j-5, which no thread reads after step j-2). The FP32 body is bound by the reciprocals (MUFU) and by how many warps hide them: holding the
 // stencil's differences in registers as the FP64 body does saves 18 of 132 packed operations per vector and
 // row but spills at 128 registers (two CTAs per SM) and was slower, 1.29 against 0.99 ms per stage at
 // 448 x 448 x 32 x 36 (1.17 at 168 registers, 12 warps per SM).
+// One phase of `bar` per row: a warp arrives when its x faces of the row are stored and its reads of the previous
+// row's are done, and waits at the next row's start, so that the row's y face hides the slowest warp.
+__device__ __forceinline__ void row_arrive(unsigned bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Every warp of the CTA arrives once per row, so the wait ends; it is bounded all the same (error word bit 3).
+__device__ __forceinline__ void row_wait(unsigned bar, int parity, unsigned* err) {
+#pragma unroll 1
+    for (int t = 0; t < (1 << 20); ++t) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred P1;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, P1;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return;
+    }
+    atomicOr(err, 8u);
+}
+
 template <bool AL, int ROWV, int XM, int YM, int MODE>
-__device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, Q* priv, int* sg, int n,
-                                              int tx, int js, int je) {
+__device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring, Q* fsm, Q* priv, int* sg, unsigned bar,
+                                              int n, int tx, int js, int je) {
     using LV = LaneVec<float>;
     constexpr bool XMIX = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
     // whole vectors, no currents: rows and c_g by cp.async (874 against 966 us per stage with the SourceTermSet
     // rates at 384 x 384 x 32 x 36, 704 against 734 without at 601 x 417 x 24 x 24; with currents 1040 against 996
     // at 448 x 448, element by element 542 against 418)
     constexpr bool ASYNC = AL && !curr;
+    // Rows divided by row_arrive / row_wait: at a barrier a warp stood 0.9 of its 7.4 cycles per instruction.
+    // Against the barrier, cases of 384 x 384 to 1024 x 1024 x 32 x 36: three steps with SourceTermSet rates 8.42 -> 8.06 ms,
+    // tides at 448 x 448 7.48 -> 7.28, self-coupled 11.53 -> 11.2, 1024 x 1024 64.1 -> 63.1; 64 x 64 x 4 x 16, one
+    // step, 112 -> 114 us (latency). Vectors copied element by element keep the barrier: 7.68 against 7.92 ms
+    // at 389 x 251 x 25 x 24.
+    constexpr bool SPLIT = AL;
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, L = p.L, CX = p.CX;
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const int tid = threadIdx.x, l = tid % L;
@@ -166,10 +195,14 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
     velo(ux0, uy0);
     Q uy1 = qz();
     vload(modr(js + 1));
-    if (XMIX && slot == 0 && act) {
-        sg[CX * L + l] = 0;
-        sg[(2 * CX + 1) * L + l] = 0;
-    }
+    if constexpr (XMIX)
+        if (act) {
+            sg[slot * L + l] = own ? codeq(ux0) : 0;           // the first row's codes
+            if (slot == 0) {
+                sg[CX * L + l] = 0;
+                sg[(2 * CX + 1) * L + l] = 0;
+            }
+        }
     __syncthreads();
     const Q* q = ring + own_off;
     Q pLy = qz(), pRy = qz();   // the two candidates of the lower y face of the current row
@@ -197,17 +230,16 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
                 if (act) put(sw, own_off, nw);
                 if (hal) put(sw, hal_off, hv);
             }
-            if constexpr (XMIX)
-                if (act) sg[(buf * (CX + 1) + slot) * L + l] = own ? codeq(ux0) : 0;
             velo(ux1, uy1);   // also waits for row j+3
             if constexpr (!ASYNC) {
                 rload(0, rl);
                 vload(rv);
             }
         }
-        __syncthreads();
+        if constexpr (!SPLIT) __syncthreads();
+        else row_wait(bar, buf, p.err);                         // the x faces of row j-1 are all stored
         if constexpr (ASYNC) {
-            if (row) {   // row j+4 into the slot of row j-4, whose readers have passed a barrier since
+            if (row) {   // row j+4 into the slot of row j-4, whose readers have arrived since
                 rload((sw + 1) & 7, rl);
                 vload(rv);
             }
@@ -236,6 +268,8 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
             }
         }
         if (!row) return false;
+        if constexpr (XMIX)
+            if (act) sg[((1 - buf) * (CX + 1) + slot) * L + l] = own ? codeq(ux1) : 0;   // for the next row
         if constexpr (FUSED) pend(js + k);
         const Q* qq = q + sq * ROWV;
         auto R = [&](int d) { return lds(qq + d * ROWV); };     // own column, row j-3+d
@@ -262,6 +296,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
             }
             ux_prev = ux0;
         }
+        if constexpr (SPLIT) row_arrive(bar);
         {
             Q Fhi, Flo;
             if constexpr (YM == POS) {
@@ -293,6 +328,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
         outoff += rs;
         return true;
     };
+    if constexpr (SPLIT) row_arrive(bar);                      // the phase the first row waits for
     for (int k = 0;; k += 2) {
         if (!step(k, std::integral_constant<int, 0>{})) break;
         if (!step(k + 1, std::integral_constant<int, 1>{})) break;
@@ -568,11 +604,13 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
 }
 
 template <typename T, bool AL, int LB, int XM, int YM, int MODE>
-__device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* smem, int* sg, int n, int tx, int js, int je) {
+__device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* smem, int* sg, unsigned bar, int n,
+                                         int tx, int js, int je) {
     if constexpr (std::is_same<T, float>::value) {
         constexpr int ROWV = XTHREADS + 5 * LB;
         Q* ring = reinterpret_cast<Q*>(smem);
-        xyw_body_ring<AL, ROWV, XM, YM, MODE>(p, ring, ring + 16 * ROWV, ring + 16 * ROWV + 4 * XTHREADS, sg, n, tx, js, je);
+        xyw_body_ring<AL, ROWV, XM, YM, MODE>(p, ring, ring + 16 * ROWV, ring + 16 * ROWV + 4 * XTHREADS, sg, bar, n, tx, js,
+                                              je);
     } else {
         D* rows = reinterpret_cast<D*>(smem);
         xyw_body<AL, XM, YM, MODE>(p, rows, rows + 2 * ROWV64, rows + 2 * ROWV64 + 4 * XTHREADS, sg, n, tx, js, je);
@@ -594,6 +632,10 @@ xyw_kernel(const WalkArgs<T> p, int seg0) {
     constexpr int N = LaneVec<T>::N;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sg[2 * (XTHREADS + MAXL)];
+    __shared__ __align__(8) unsigned long long row_bar;
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(&row_bar);
+    if (std::is_same<T, float>::value && threadIdx.x == 0)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(blockDim.x / 32) : "memory");
     int b = blockIdx.x;
     const int n = b % p.Np;
     b /= p.Np;
@@ -625,7 +667,7 @@ xyw_kernel(const WalkArgs<T> p, int seg0) {
     // component's sign depends on the current. Against the four uniform bodies and one general body: 407 against
     // 431 us per stage at 389 x 251 x 25 x 24 FP32, 1041 against 1068 at 320 x 320 x 32 x 36 FP64.
 #define RPL_BODY(X, Y) \
-    if (xm == X && ym == Y) return run_body<T, AL, LB, X, Y, MODE>(p, smem, sg, n, tx, js, je)
+    if (xm == X && ym == Y) return run_body<T, AL, LB, X, Y, MODE>(p, smem, sg, bar, n, tx, js, je)
     RPL_BODY(POS, POS);
     RPL_BODY(POS, NEG);
     RPL_BODY(NEG, POS);

@@ -75,6 +75,19 @@ def test_sources_match_oracle(oracle_mod, shape, precision, transport, sources):
     assert rel_l2(run(w, precision), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL[precision]
 
 
+@pytest.mark.parametrize("shape", [(3, 5, 4, 3), (31, 6, 32, 4), (64, 130, 8, 5), (40, 9, 64, 3), (255, 5, 4, 4)])
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+def test_whole_vectors_fp32_match_oracle_and_repeat(oracle_mod, shape, transport):
+    """Rows handed on without a CTA barrier (whole FP32 lane vectors): one to eight warps per CTA, segments of one row
+    upwards, uniform and mixed signs; the oracle's result, and the same bits on every run."""
+    for current in (0.05, 3.0):
+        w = workload(shape, current, transport=transport)
+        first = run(w, "fp32")
+        assert rel_l2(first, oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL["fp32"]
+        for _ in range(3):
+            assert np.array_equal(run(w, "fp32"), first)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_model_without_room_for_the_planes_takes_the_column_kernel(precision):
     """A memory limit that holds the model but not the two-pass stage's c_g plane: same result."""
