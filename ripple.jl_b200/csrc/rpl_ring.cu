@@ -263,8 +263,9 @@ struct Lane {
     }
 };
 
-// Shared memory of ring_kernel in 16-byte slots per thread: the window ring twice, then S and N0 of two steps.
-constexpr int WIN = 16, SLOTS = WIN + 4;
+// Shared memory of ring_kernel in 16-byte slots per thread: the window ring twice, then S and N0 of two steps. Behind
+// them the direction table of the CTA's range, TABLE_NP entries (32 KiB) at most.
+constexpr int WIN = 16, SLOTS = WIN + 4, TABLE_NP = 1024;
 
 template <typename T, bool AL, bool BUNDLE, bool RATES>
 __global__ void __launch_bounds__(RTHREADS, BUNDLE ? 2 : 4)
@@ -276,13 +277,13 @@ ring_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
     V* slot = reinterpret_cast<V*>(smem) + threadIdx.x;
     Trig* trig = reinterpret_cast<Trig*>(smem + SLOTS * RTHREADS * 16);
     const int Nk = p.Nk, Np = p.Np;
-    for (int n = threadIdx.x; n < Np; n += RTHREADS) trig[n] = Vel<T>::trig(p, n);
+    const int n0 = blockIdx.y * per_part, n1 = min(n0 + per_part, Np);
+    for (int n = n0 + threadIdx.x; n < n1; n += RTHREADS) trig[n - n0] = Vel<T>::trig(p, n);
     __syncthreads();
     const int64_t slice = (int64_t)p.Nx * p.Ny * Nk;
     const Lane<T> me(p);
     const int left = me.left;
     const Edges edge{me.m0, Nk};
-    const int n0 = blockIdx.y * per_part, n1 = min(n0 + per_part, Np);
     const T* own = p.Nin + me.home;
     auto window = [&](int s, const T* src) {   // a direction's slice into ring slot s
         copy_async<AL>(slot + s * RTHREADS, src, left);
@@ -329,7 +330,7 @@ ring_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
         V rate = LV::zero();
         if (RATES) rate = ldv<AL>(p.rates + off, left);
         V ck, cp;
-        vel.at(trig[n], ck, cp);
+        vel.at(trig[n - n0], ck, cp);
         const int vk = __all_sync(FULL, all_pos(ck)) ? 1 : (__all_sync(FULL, all_neg(ck)) ? 2 : 0);
         const V fk = qmuls(kappa_flux(c, ck, vk, edge, me.l, p.L, me.lane), p.dk_inv);
         const int vp = __all_sync(FULL, all_pos(cp)) ? 1 : (__all_sync(FULL, all_neg(cp)) ? 2 : 0);
@@ -403,11 +404,14 @@ __global__ void __launch_bounds__(RTHREADS, 4) bundle_kernel(const WalkArgs<T> p
 
 template <typename T, bool AL>
 cudaError_t launch_al(const WalkArgs<T>& a, const StageParams& p, bool refract, bool bundle, cudaStream_t s) {
+    if (a.L < 1) return cudaErrorInvalidValue;   // no lane geometry (walk_supported)
     const int64_t P = (int64_t)a.Nx * (a.j_hi - a.j_lo), per = (RTHREADS / 32) * (32 / a.L);
     const unsigned blocks = (unsigned)((P + per - 1) / per);
     // ranges of the ring: one unless that leaves the GPU without eight CTAs per SM, then as many as that
-    // takes, of at least three directions each (a range pays a 7-deep window and one more face)
-    const int64_t parts = std::max<int64_t>(1, std::min<int64_t>((8 * 148 + blocks - 1) / blocks, a.Np / 3));
+    // takes, of at least three directions each (a range pays a 7-deep window and one more face); never more
+    // directions in a range than its table holds
+    const int64_t parts = std::max<int64_t>({1, std::min<int64_t>((8 * 148 + blocks - 1) / blocks, a.Np / 3),
+                                             (a.Np + TABLE_NP - 1) / TABLE_NP});
     const int per_part = (int)((a.Np + parts - 1) / parts);
     const dim3 grid(blocks, (unsigned)((a.Np + per_part - 1) / per_part));
     const bool rates = a.rates != nullptr;
@@ -419,7 +423,7 @@ cudaError_t launch_al(const WalkArgs<T>& a, const StageParams& p, bool refract, 
         k<<<grid, RTHREADS, smem, s>>>(a, p, per_part);
         return cudaGetLastError();
     };
-    const size_t ring = SLOTS * RTHREADS * 16 + a.Np * sizeof(typename Vel<T>::Trig);
+    const size_t ring = SLOTS * RTHREADS * 16 + per_part * sizeof(typename Vel<T>::Trig);
     if (refract && bundle) return rates ? go(ring_kernel<T, AL, true, true>, ring) : go(ring_kernel<T, AL, true, false>, ring);
     if (refract) return rates ? go(ring_kernel<T, AL, false, true>, ring) : go(ring_kernel<T, AL, false, false>, ring);
     const size_t staged = DEPTH * 3 * RTHREADS * 16;

@@ -593,8 +593,12 @@ __global__ void __launch_bounds__(CPB * L, MINB) kp_kernel(const TileArgs p) {
 // Second pass of an intrinsic stage with the bundle (SRC 1) or the learned (SRC 2) sources, after the
 // y-walk x/y pass stored S = fx + fy: one thread per (cell, kappa pair) walking the phi ring with the
 // cell's wind constants and its bins' constants loaded once; G = -S, the sources and the stage update
-// as the tile body (G = -(fx + fy) there).
-template <int L, int CPB, int MINB, int SRC>
+// as the tile body (G = -(fx + fy) there). STAGED: the directions' (cos, sin) in shared memory, not behind the
+// streaming loads in L1; more directions than KS_TABLE_NP (8 KiB) are read from memory (a choice inside the
+// kernel, by the count, cost 6% of a 768 x 768 x 32 x 36 step: 31.6 against 29.9 ms for two).
+constexpr int KS_TABLE_NP = 1024;
+
+template <int L, int CPB, int MINB, int SRC, bool STAGED>
 __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
     static_assert(SRC == 1 || SRC == 2, "bundle or learned sources");
     const float* S = p.sxy;   // may be Nout: each element is read, then written, by one thread
@@ -602,9 +606,11 @@ __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
     const float* N0 = p.N0;
     float* Nout = p.Nout;
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, Np = p.Np;
-    extern __shared__ float2 s_cs[];   // the directions' (cos, sin): not behind the streaming loads in L1
-    for (int n = threadIdx.x; n < Np; n += CPB * L) s_cs[n] = __ldg(p.cs32 + n);
-    __syncthreads();
+    extern __shared__ float2 s_cs[];
+    if constexpr (STAGED) {
+        for (int n = threadIdx.x; n < Np; n += CPB * L) s_cs[n] = __ldg(p.cs32 + n);
+        __syncthreads();
+    }
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const int64_t P = (int64_t)Nx * (p.j_hi - p.j_lo);
     const int tid = threadIdx.x, l = tid % L;
@@ -639,7 +645,7 @@ __global__ void __launch_bounds__(CPB * L, MINB) ks_kernel(const TileArgs p) {
         if (n + 1 < Np) fetch(off + slice);
         float2 G = mul2(f2(-1.f), sxy);
         if (plain_src) {
-            const float2 cs = s_cs[n];
+            const float2 cs = STAGED ? s_cs[n] : __ldg(p.cs32 + n);
             const bool with = fmaf(cs.x, wc.cu, cs.y * wc.su) > 0.0f;
             G.x += source32(p, wc, wb0, cs.x, cs.y, c.x, grow0 && with);
             G.y += source32(p, wc, wb1, cs.x, cs.y, c.y, grow1 && with);
@@ -729,7 +735,7 @@ cudaError_t launch_variant(const TileArgs& a, int tiles, cudaStream_t s) {
 
 // Two-pass refraction stage: the x/y pass (the y-walk; staged tiles with RPL_PASS_A=tiles or without velocity
 // planes), then the ring walk with four kappa bins per lane without the bundle or learned sources, else (or
-// with RPL_PASS_B=pairs) the pair kernel in 256-thread CTAs.
+// with RPL_PASS_B=pairs, or without the walk's geometry) the pair kernel in 256-thread CTAs.
 template <int L, int SRC>
 cudaError_t launch_split(const Handle& h, const StageParams& p, const TileArgs& a, const WalkArgs<float>& w,
                          cudaStream_t s) {
@@ -746,7 +752,7 @@ cudaError_t launch_split(const Handle& h, const StageParams& p, const TileArgs& 
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
-    if ((SRC == 0 || SRC == 3) && !h.pass_b_pairs) return launch_ring<float>(w, p, true, false, s);
+    if ((SRC == 0 || SRC == 3) && !h.pass_b_pairs && w.L > 0) return launch_ring<float>(w, p, true, false, s);
     const int64_t cells = (int64_t)a.Nx * (a.j_hi - a.j_lo);
     // the per-cell source constants of the bundle and the learned source need registers: two CTAs per SM
     constexpr int BMINB = (SRC == 1 || SRC == 2) ? 2 : 3;
@@ -774,8 +780,11 @@ cudaError_t launch_L(const Handle& h, const StageParams& p, const TileArgs& a, c
         constexpr int CPB = 256 / L;
         const int64_t cells = (int64_t)a.Nx * (a.j_hi - a.j_lo);
         const unsigned blocks = (unsigned)((cells + CPB - 1) / CPB);
-        if (src == 1) ks_kernel<L, CPB, 3, 1><<<blocks, CPB * L, a.Np * sizeof(float2), s>>>(a);
-        else ks_kernel<L, CPB, 2, 2><<<blocks, CPB * L, a.Np * sizeof(float2), s>>>(a);
+        const bool staged = a.Np <= KS_TABLE_NP;
+        const size_t table = staged ? a.Np * sizeof(float2) : 0;
+        auto k = src == 1 ? (staged ? ks_kernel<L, CPB, 3, 1, true> : ks_kernel<L, CPB, 3, 1, false>)
+                          : (staged ? ks_kernel<L, CPB, 2, 2, true> : ks_kernel<L, CPB, 2, 2, false>);
+        k<<<blocks, CPB * L, table, s>>>(a);
         return cudaGetLastError();
     }
     if (src == 3) return launch_variant<L, 3>(a, tiles, s);

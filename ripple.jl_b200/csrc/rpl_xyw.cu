@@ -67,10 +67,9 @@ cudaError_t launch_xyw(const WalkArgs<double>& a, const WalkGeom& g, cudaStream_
 }  // namespace
 
 bool walk_supported(const rpl_desc& d) {
-    // at most 32 lanes per cell and, for the ring walk's direction table in shared memory, 1024 directions;
-    // offsets within one direction slice are 32-bit
+    // at most 32 lanes per cell; offsets within one direction slice are 32-bit
     return (d.transport == RPL_TRANSPORT_REFRACTION || d.transport == RPL_TRANSPORT_INTRINSIC) && d.Nk <= 64 &&
-           d.Np <= 1024 && d.Nx * d.Ny * d.Nk < (int64_t)1 << 31 && d.Nx >= 3 && d.Ny >= 3 &&
+           d.Nx * d.Ny * d.Nk < (int64_t)1 << 31 && d.Nx >= 3 && d.Ny >= 3 &&
            (d.transport != RPL_TRANSPORT_REFRACTION || d.Np >= 3);
 }
 
