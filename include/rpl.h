@@ -87,7 +87,9 @@ typedef struct rpl_desc {
     double depth_constant;
     const double* depth_field;  /* Nx*Ny */
     double gravity;             /* 9.81 in the reference */
-    int64_t memory_limit_bytes; /* 0: no limit; else creation fails with RPL_ERR_OOM above it */
+    int64_t memory_limit_bytes; /* 0: no limit; else creation fails with RPL_ERR_OOM above it, as does a later
+                                   call that needs more; tables that only save time are taken where they fit and
+                                   given up for such a call (unless a stream capture has recorded their use) */
     const double* xspacings;    /* Nx cell widths Δx(i) and Ny cell heights Δy(j): the total action sums */
     const double* yspacings;    /* m0(i,j)·Δx(i)·Δy(j) (diagnostic_operations.jl:492-503); NULL: dx, dy */
 } rpl_desc;

@@ -64,7 +64,7 @@ std::string check_faces(const char* name, const double* c, const double* f, int6
 template <typename T>
 cudaError_t dalloc(Handle* h, T** p, size_t count) {
     const size_t bytes = count * sizeof(T);
-    cudaError_t e = cudaMalloc((void**)p, bytes ? bytes : 8);
+    cudaError_t e = rpl::device_alloc(h, (void**)p, bytes ? bytes : 8);
     if (e == cudaSuccess) h->bytes += (int64_t)bytes;
     return e;
 }
@@ -85,7 +85,47 @@ void free_all(Handle* h) {
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
 
+// Releases the velocity planes once the stages in flight have read them; false where there are none to release
+// or a captured graph may use them.
+bool drop_planes(Handle* h) {
+    if (!h->d_vel) return false;
+    rpl::pin_planes(*h, h->stream);   // no synchronisation of a capturing stream
+    if (h->vel_pinned || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+    if (cudaFree(h->d_vel) != cudaSuccess) return false;
+    cudaFree(h->d_rmax);
+    h->d_vel = nullptr;
+    h->d_rmax = nullptr;
+    h->bytes -= h->vel_bytes;
+    h->vel_bytes = 0;
+    return true;
+}
+
 }  // namespace
+
+bool rpl::make_room(Handle* h, int64_t extra) {
+    const int64_t limit = h->desc.memory_limit_bytes;
+    if (limit <= 0 || h->bytes + extra <= limit) return true;
+    return h->bytes - h->vel_bytes + extra <= limit && drop_planes(h);
+}
+
+cudaError_t rpl::device_alloc(Handle* h, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && drop_planes(h)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+void rpl::pin_planes(const Handle& h, cudaStream_t s) {
+    if (!h.d_vel || h.vel_pinned) return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // the legacy stream beside another stream's capture
+        cudaGetLastError();
+        h.vel_pinned = true;
+    }
+    if (st != cudaStreamCaptureStatusNone) h.vel_pinned = true;
+}
 
 // Releases the prescribed-currents state (Q grid, weight tables, the device copy of u and v).
 void rpl::free_currents(Handle* h) {
@@ -397,17 +437,20 @@ int rpl_create(const rpl_desc* d, rpl_handle** out) {
     TRY(dalloc(h, &h->d_coef, 8 * c3));
     TRY(dalloc(h, &h->d_cell32, 8 * P));
     TRY(dalloc(h, &h->d_bin32, 8 * d->Nk));
+    TRY(dalloc(h, &h->d_tab32, 6 * d->Np + 3 * nb));
     if (rpl::walk_supported(*d)) h->walk = rpl::walk_geometry(*d);
     if (rpl::walk_supported(*d) && !h->force_column_kernel && !(h->pass_a_tiles && rpl::tile32_supported(*h))) {
         // the two-pass stage: velocity planes (intrinsic: c_g only) and upwind ratios. A model whose memory
-        // limit or device has no room for them takes the kernels that read the coefficient records.
+        // limit or device has no room for them, now or at a later call (make_room, device_alloc), takes the kernels
+        // that read the coefficient records.
         h->vel_regions = (int64_t)h->walk.tiles_x * ((d->Ny + h->walk.seg - 1) / h->walk.seg);
         const int64_t plane = (d->transport == RPL_TRANSPORT_REFRACTION ? 3 : 1) * c3 * (int64_t)elem;
         const int64_t ratios = 2 * h->vel_regions * d->Nk * 4;
         if (!(d->memory_limit_bytes > 0 && need + plane + ratios > d->memory_limit_bytes)) {
             if (cudaMalloc(&h->d_vel, plane) == cudaSuccess &&
                 cudaMalloc((void**)&h->d_rmax, ratios) == cudaSuccess) {
-                h->bytes += plane + ratios;
+                h->vel_bytes = plane + ratios;
+                h->bytes += h->vel_bytes;
             } else {
                 cudaGetLastError();
                 if (h->d_vel) cudaFree(h->d_vel);
@@ -435,7 +478,6 @@ int rpl_create(const rpl_desc* d, rpl_handle** out) {
             tab32[4 * d->Np + 2 * nb + 2 * n] = (float)cosp[n];
             tab32[4 * d->Np + 2 * nb + 2 * n + 1] = (float)sinp[n];
         }
-        TRY(dalloc(h, &h->d_tab32, tab32.size()));
         TRY(cudaMemcpyAsync(h->d_tab32, tab32.data(), tab32.size() * 4, cudaMemcpyHostToDevice, s));
         TRY(cudaStreamSynchronize(s));
     }
@@ -486,7 +528,7 @@ int rpl_set_currents(rpl_handle* hh, int64_t Nz, const double* z_faces, int32_t 
     RPL_CUDA(cudaStreamSynchronize(s));
     rpl::free_pm(h);  // prescribed currents replace a pseudomomentum coupling
     rpl::free_currents(h);
-    if (d.memory_limit_bytes > 0 && h->bytes + extra > d.memory_limit_bytes)
+    if (!rpl::make_room(h, extra))
         return fail(RPL_ERR_OOM, "currents need " + std::to_string(extra) + " more device bytes, above the memory limit");
     h->currents_set = false;
     if (!h->d_coupling) RPL_CUDA(dalloc(h, &h->d_coupling, 8 * c3));
@@ -886,8 +928,8 @@ int rpl_tendency(rpl_handle* hh, double* G, int32_t layout) {
     if ((st = check_step_args(h, 1.0))) return st;
     cudaStream_t s = h->stream;
     double *dG = nullptr, *dGx = nullptr;
-    RPL_CUDA(cudaMalloc(&dG, h->units * 8));
-    cudaError_t e = cudaMalloc(&dGx, h->units * 8);
+    RPL_CUDA(rpl::device_alloc(h, (void**)&dG, h->units * 8));
+    cudaError_t e = rpl::device_alloc(h, (void**)&dGx, h->units * 8);
     if (e == cudaSuccess && h->has_sources && h->src.wind_kind != RPL_WIND_NONE) {
         e = rpl::launch_wind(*h, h->time, s);
         if (e == cudaSuccess && h->src.stress_cap) e = rpl::launch_stress_factor(*h, h->N, s);

@@ -138,7 +138,8 @@ struct Handle {
     void* d_vel = nullptr;         // y-walk x/y pass: planes U_x, U_y, c_g per (i,j,m) in the state's type
                                    // (intrinsic transport: c_g only); null: the model takes other kernels
     unsigned int* d_rmax = nullptr;  // y-walk x/y pass: per region, axis and bin the upwind ratio maxima
-    int64_t vel_regions = 0;
+    int64_t vel_regions = 0, vel_bytes = 0;
+    mutable bool vel_pinned = false;   // a captured graph may hold the planes' addresses: never given up
     WalkGeom walk;
     // learned source (rpl_learned.cu)
     rpl_mlp* learned = nullptr;
@@ -237,6 +238,16 @@ void free_smooth(Handle* h);
 // SourceTermSet rates of the action Nin into d_lin_rates; release of their buffers (rpl_terms.cu).
 cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s);
 void free_terms(Handle* h);
+
+// ---- device memory (rpl_api.cu) ----
+// The velocity planes are an optimisation: where a later request would not fit the handle's memory limit, or the
+// device, with them, they are given up and the stages take the kernels that read the coefficient records.
+// Whether `extra` more device bytes fit the handle's memory limit.
+bool make_room(Handle* h, int64_t extra);
+// cudaMalloc for a handle's buffers (the caller counts them in h->bytes).
+cudaError_t device_alloc(Handle* h, void** p, size_t bytes);
+// Notes a stream capture: the graph keeps the planes' addresses. Called by every launch that passes them on.
+void pin_planes(const Handle& h, cudaStream_t s);
 
 // Sets the thread-local message rpl_last_error() returns (rpl_api.cu).
 void set_last_error(const std::string& msg);

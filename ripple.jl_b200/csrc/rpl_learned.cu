@@ -233,9 +233,9 @@ int rpl_set_learned_source(rpl_handle* hh, rpl_mlp* m, const float* lo, const fl
     const int64_t rows = (h->cells + 127) / 128 * 128;
     const size_t nbound = (size_t)2 * (nb + 4) + 2 * nb;  // input lo, hi, output lo, hi
     const size_t need = rows * nb * (2 + 4) + rows * 16 + h->cells * 4 + nbound * 4;
-    if (h->desc.memory_limit_bytes > 0 && h->bytes + (int64_t)need > h->desc.memory_limit_bytes)
+    if (!rpl::make_room(h, (int64_t)need))
         return rpl::lfail(RPL_ERR_OOM, "the learned source's buffers would exceed memory_limit_bytes");
-    auto al = [&](auto** p, size_t bytes) { return cudaMalloc((void**)p, bytes); };
+    auto al = [&](auto** p, size_t bytes) { return rpl::device_alloc(h, (void**)p, bytes); };
     if ((e = al(&h->d_lx, rows * nb * 2)) != cudaSuccess || (e = al(&h->d_le, rows * 16)) != cudaSuccess ||
         (e = al(&h->d_lr, rows * nb * 4)) != cudaSuccess ||
         (e = al(&h->d_lflag, h->cells * sizeof(unsigned int))) != cudaSuccess ||

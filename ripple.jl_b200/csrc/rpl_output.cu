@@ -104,10 +104,10 @@ int rpl_snapshot_async(rpl_handle* hh, void* host, int32_t dtype) {
             h->d_snap = nullptr;
             h->snap_bytes = 0;
         }
-        if (h->desc.memory_limit_bytes > 0 && h->bytes + bytes > h->desc.memory_limit_bytes)
+        if (!rpl::make_room(h, bytes))
             return ofail(RPL_ERR_OOM, "the snapshot staging buffer (" + std::to_string(bytes) +
                                           " bytes) would exceed the memory limit");
-        e = cudaMalloc(&h->d_snap, bytes);
+        e = rpl::device_alloc(h, &h->d_snap, bytes);
         if (e != cudaSuccess) {
             h->d_snap = nullptr;
             return ocuda(e, "snapshot staging buffer");

@@ -295,7 +295,7 @@ extern "C" int rpl_set_pseudomomentum(rpl_handle* hh, int64_t Nz, const double* 
     const int64_t f32_bytes = f32 ? cols * Nk * Nk * 4 + 2 * Nk * Np * 4 : 0;
     const int64_t extra = table_bytes + moment_bytes + f32_bytes + (h->d_coupling ? 0 : 8 * c3 * 8) +
                           (h->d_U ? 0 : 4 * c3 * 8);
-    if (d.memory_limit_bytes > 0 && h->bytes + extra > d.memory_limit_bytes)
+    if (!rpl::make_room(h, extra))
         return pm_fail(RPL_ERR_OOM, "pseudomomentum tables need " + std::to_string(extra) +
                                         " more device bytes, above the memory limit");
     cudaStream_t s = h->stream;
@@ -305,19 +305,20 @@ extern "C" int rpl_set_pseudomomentum(rpl_handle* hh, int64_t Nz, const double* 
     rpl::free_pm(h);
     rpl::free_currents(h);
     if (!h->d_coupling) {
-        e = cudaMalloc(&h->d_coupling, 8 * c3 * sizeof(double));
+        e = rpl::device_alloc(h, (void**)&h->d_coupling, 8 * c3 * sizeof(double));
         if (e != cudaSuccess) return pm_fail(RPL_ERR_OOM, "pseudomomentum coupling: device allocation failed");
         h->bytes += 8 * c3 * 8;
     }
     if (!h->d_U) {
-        e = cudaMalloc(&h->d_U, 4 * c3 * sizeof(double));
+        e = rpl::device_alloc(h, (void**)&h->d_U, 4 * c3 * sizeof(double));
         if (e != cudaSuccess) return pm_fail(RPL_ERR_OOM, "pseudomomentum coupling: device allocation failed");
         h->bytes += 4 * c3 * 8;
     }
-    e = cudaMalloc(&h->d_pm_overlap, table_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_pm_moments, moment_bytes);
-    if (e == cudaSuccess && f32) e = cudaMalloc(&h->d_pm_overlap32, cols * Nk * Nk * 4);
-    if (e == cudaSuccess && f32) e = cudaMalloc(&h->d_pm_moments32, 2 * Nk * Np * 4);
+    auto alloc = [&](auto** p, int64_t bytes) { return rpl::device_alloc(h, (void**)p, bytes); };
+    e = alloc(&h->d_pm_overlap, table_bytes);
+    if (e == cudaSuccess) e = alloc(&h->d_pm_moments, moment_bytes);
+    if (e == cudaSuccess && f32) e = alloc(&h->d_pm_overlap32, cols * Nk * Nk * 4);
+    if (e == cudaSuccess && f32) e = alloc(&h->d_pm_moments32, 2 * Nk * Np * 4);
     if (e == cudaSuccess) {
         h->bytes += table_bytes + moment_bytes + f32_bytes;
         h->pm_cols = cols;
@@ -343,8 +344,8 @@ extern "C" int rpl_set_pseudomomentum(rpl_handle* hh, int64_t Nz, const double* 
             mom[Nk * Np + m + Nk * n] = radial * (std::cos(p1) - std::cos(p2));
         }
     double *dz = nullptr, *dq = nullptr;
-    e = cudaMalloc(&dz, (Nz + 1) * 8);
-    if (e == cudaSuccess && cols > 1) e = cudaMalloc(&dq, P * 8);
+    e = alloc(&dz, (Nz + 1) * 8);
+    if (e == cudaSuccess && cols > 1) e = alloc(&dq, P * 8);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, z_faces, (Nz + 1) * 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && dq) e = cudaMemcpyAsync(dq, q_depth_field, P * 8, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_pm_moments, mom.data(), moment_bytes, cudaMemcpyHostToDevice, s);

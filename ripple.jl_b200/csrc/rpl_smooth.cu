@@ -294,9 +294,9 @@ extern "C" int rpl_set_propagation_smoothing(rpl_handle* hh, int32_t kind, doubl
     const size_t elem = h->precision == RPL_FP64 ? 8 : 4;
     const int64_t Nk = h->desc.Nk, Np = h->desc.Np, ntab = 2 * Nk + 2 * Np;
     const int64_t bytes = ntab * 8 + 9 * Nk * Np * (int64_t)elem + Nk * Np * 4;
-    if (h->desc.memory_limit_bytes > 0 && h->bytes + bytes > h->desc.memory_limit_bytes)
+    if (!rpl::make_room(h, bytes))
         return fail(RPL_ERR_OOM, "SpatialAveraging tables would exceed the memory limit");
-    e = cudaMalloc(&h->d_smooth, bytes);
+    e = rpl::device_alloc(h, &h->d_smooth, bytes);
     if (e != cudaSuccess) {
         h->d_smooth = nullptr;
         cudaGetLastError();

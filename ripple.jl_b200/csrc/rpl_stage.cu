@@ -478,6 +478,7 @@ cudaError_t launch_walk(const Handle& h, const StageParams& p, const void* Nin, 
 
 cudaError_t launch_stage(const Handle& h, const StageParams& p, const void* Nin, const void* N0, void* Nout,
                          cudaStream_t s) {
+    pin_planes(h, s);
     if (h.precision == RPL_FP64) {
         if (h.d_vel) return launch_walk<double>(h, p, Nin, N0, Nout, s);
         return launch_impl<double, false>(h, p, Nin, N0, Nout, nullptr, s);

@@ -628,13 +628,12 @@ extern "C" int rpl_set_source_terms(rpl_handle* hh, const rpl_source_term* terms
     }
     const int64_t rate_bytes = h->units * (int64_t)h->elem, tab_bytes = (int64_t)host.size() * 8;
     const int64_t col_bytes = count <= 4 ? P * count * (int64_t)sizeof(double2) : 0;
-    const int64_t limit = d.memory_limit_bytes;
-    if (limit > 0 && h->bytes + rate_bytes + tab_bytes + col_bytes > limit)
+    if (!make_room(h, rate_bytes + tab_bytes + col_bytes))
         return fail(RPL_ERR_OOM, "source terms need " + std::to_string(rate_bytes + tab_bytes + col_bytes) +
                                      " more device bytes, above the memory limit");
-    e = cudaMalloc(&h->d_lin_rates, rate_bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_terms, tab_bytes);
-    if (e == cudaSuccess && col_bytes) e = cudaMalloc((void**)&h->d_tcol, col_bytes);
+    e = device_alloc(h, &h->d_lin_rates, rate_bytes);
+    if (e == cudaSuccess) e = device_alloc(h, (void**)&h->d_terms, tab_bytes);
+    if (e == cudaSuccess && col_bytes) e = device_alloc(h, (void**)&h->d_tcol, col_bytes);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h->d_terms, host.data(), tab_bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);

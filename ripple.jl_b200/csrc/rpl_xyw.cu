@@ -92,6 +92,7 @@ WalkGeom walk_geometry(const rpl_desc& d) {
 
 cudaError_t launch_vel(const Handle& h, cudaStream_t s) {
     if (!h.d_vel) return cudaSuccess;
+    pin_planes(h, s);
     const rpl_desc& d = h.desc;
     const int64_t c3 = d.Nx * d.Ny * d.Nk;
     const int per_tile = h.walk.CX - 1;

@@ -50,3 +50,66 @@ def test_ring_split_for_its_table_alone(monkeypatch):
         m.close()
     assert not torch.equal(out[""], N)
     assert torch.equal(out[""], out["pairs"])
+
+
+REFRACTION = ("currents", "pseudomomentum", "refraction_terms", "averaging")
+
+
+def bare_model(kind, precision, Nk, **kw):
+    """A model of 24 x 20 cells and the call that asks for more device memory after its creation."""
+    w = workload((24, 20, Nk, 48), 0.3, None, "refraction" if kind in REFRACTION else "intrinsic")
+    w.dt = 0.02 * 8 / 48
+    if kind == "pseudomomentum":
+        w.velocities = rp.PseudomomentumVelocities()
+    if kind in ("terms", "refraction_terms"):
+        w.sources = terms()
+    if kind == "averaging":
+        w.propagation_smoothing = rp.SpatialAveraging()
+    m = w.model(precision, **kw)
+    if kind == "snapshot":
+        from ripple_b200 import output
+        output.snapshot_async(m)
+        output.snapshot_wait(m)
+    return w, m
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("Nk", [8, 25])
+@pytest.mark.parametrize("kind", ["currents", "pseudomomentum", "terms", "refraction_terms", "averaging", "snapshot"])
+def test_planes_are_given_up_for_what_a_later_call_needs(kind, precision, Nk):
+    """A memory limit that holds the model and the planes, or the model and what a later call asks for, but not all
+    three: the call is accepted, the planes go, and the other stage kernels give the same result (rounding apart).
+    Without room for the call itself it is refused."""
+    w, full = bare_model(kind, precision, Nk)
+    total, cells, e = full.device_bytes(), 480, 8 if precision == "fp64" else 4
+    planes = cells * Nk * e * (3 if kind in REFRACTION else 1)
+    _, small = bare_model(kind, precision, Nk, memory_limit_bytes=total - 1)
+    assert small.device_bytes() <= total - planes
+    with pytest.raises(rp.RplError):
+        bare_model(kind, precision, Nk, memory_limit_bytes=small.device_bytes() - 1)
+    rp.time_step(full, w.dt, 2)
+    rp.time_step(small, w.dt, 2)
+    assert rel_l2(small.action.interior(), full.action.interior()) <= (1e-13 if precision == "fp64" else 1e-6)
+
+
+def test_captured_planes_stay():
+    """Steps recorded in a CUDA graph hold the planes' addresses: a later call over the limit is refused, and the graph
+    still gives the steps' result."""
+    import torch
+    w = workload((24, 20, 25, 48), 0.3, None, "intrinsic")
+    ref = w.model("fp64")
+    m = w.model("fp64", memory_limit_bytes=ref.device_bytes() + 8 * w.units - 1)
+    s = torch.cuda.Stream()
+    _lib.check(m._lib.rpl_set_stream(m.handle, ctypes.c_void_p(s.cuda_stream)))
+    rp.time_step(m, w.dt, 1)                       # kernels loaded before the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        _lib.check(m._lib.rpl_step_async(m.handle, w.dt, 1))
+    before = m.device_bytes()
+    out = np.empty(w.N0.shape, order="F")
+    assert m._lib.rpl_snapshot_async(m.handle, out.ctypes.data_as(ctypes.c_void_p), _lib.RPL_F64) == _lib.RPL_ERR_OOM
+    assert m.device_bytes() == before
+    graph.replay()
+    torch.cuda.synchronize()
+    rp.time_step(ref, w.dt, 2)
+    assert np.array_equal(m.action.interior(), ref.action.interior())
