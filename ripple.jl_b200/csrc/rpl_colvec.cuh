@@ -61,7 +61,9 @@ template <typename A> __device__ __forceinline__ void stage_table(A* dst, const 
     }
 }
 
-// Most bytes of tables a CTA stages; a model with more takes the kernels' global-memory tables.
+// Most bytes of tables a CTA stages; a model with more takes the kernels' global-memory tables. Every launch allows its
+// kernel this much dynamic shared memory, whatever the model needs of it: the attribute belongs to the kernel, not to
+// the launch, and handles launch from several threads.
 constexpr size_t kTableBytes = 200 * 1024;
 
 }  // namespace rpl

@@ -193,7 +193,7 @@ cudaError_t pm_velocity(const Handle& h, const void* Nin, const A* moments, cons
     auto k = !staged ? pm_velocity_kernel<T, A, false, false>
                      : (Nk % VN == 0 ? pm_velocity_kernel<T, A, true, true> : pm_velocity_kernel<T, A, false, true>);
     const size_t smem = mom + (staged ? tab : 0);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(PM_WARPS * cpw)), 148 * 4);
     k<<<blocks, PM_WARPS * 32, smem, s>>>((const T*)Nin, P, Nk, Np, moments, moments + nb, overlap, h.pm_cols > 1, U, U + c3);

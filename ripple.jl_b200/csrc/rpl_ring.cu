@@ -416,8 +416,9 @@ cudaError_t launch_al(const WalkArgs<T>& a, const StageParams& p, bool refract, 
     const dim3 grid(blocks, (unsigned)((a.Np + per_part - 1) / per_part));
     const bool rates = a.rates != nullptr;
     auto go = [&](auto k, size_t smem) {
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > 48 * 1024) {   // the most any model takes: the attribute is the kernel's, shared by all threads
+            constexpr int most = SLOTS * RTHREADS * 16 + TABLE_NP * (int)sizeof(typename Vel<T>::Trig);
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
             if (e != cudaSuccess) return e;
         }
         k<<<grid, RTHREADS, smem, s>>>(a, p, per_part);

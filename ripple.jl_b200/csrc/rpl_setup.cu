@@ -612,7 +612,7 @@ cudaError_t launch_diagnostics(const Handle& h, const void* Nin, cudaStream_t s,
         auto k = smem > kTableBytes ? diag_kernel<T, false, ALL, false>
                                     : (al ? diag_kernel<T, true, ALL, true> : diag_kernel<T, false, ALL, true>);
         const size_t used = smem > kTableBytes ? 0 : smem;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes);
         if (e != cudaSuccess) return e;
         const int64_t cpw = 32 / std::min<int64_t>((d.Nk + ColVec<T>::N - 1) / ColVec<T>::N, 32);
         const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(16 * cpw)), 148 * 2);

@@ -513,7 +513,7 @@ cudaError_t launch_terms(const Handle& h, const void* Nin, cudaStream_t s) {
             const size_t smem = 4 * (size_t)table_stride<T>((int)a.Nk) * a.Np * 8, used = smem > kTableBytes ? 0 : smem;
             auto k = !used ? terms_cols_kernel<T, false, false>
                            : (a.Nk % VN == 0 ? terms_cols_kernel<T, true, true> : terms_cols_kernel<T, false, true>);
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)used);
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes);
             if (e != cudaSuccess) return e;
             const int64_t per = 16 * (32 / std::min<int64_t>((a.Nk + VN - 1) / VN, 32));
             k<<<(unsigned)std::min<int64_t>((a.P + per - 1) / per, 148 * 2), 256, used, s>>>(in, a, h.d_tcol);

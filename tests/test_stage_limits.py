@@ -113,3 +113,38 @@ def test_captured_planes_stay():
     torch.cuda.synchronize()
     rp.time_step(ref, w.dt, 2)
     assert np.array_equal(m.action.interior(), ref.action.interior())
+
+
+@pytest.mark.parametrize("kind", ["diagnostics", "terms", "pseudomomentum"])
+def test_models_of_different_sizes_launch_from_two_threads(kind):
+    """Kernels whose shared-memory tables differ with the spectrum, launched by two threads at once: no launch is refused."""
+    import threading
+    import torch
+
+    def make(Np):
+        w = workload((8, 8, 32, Np), 0.1, terms() if kind == "terms" else None,
+                     "refraction" if kind == "pseudomomentum" else "intrinsic")
+        if kind == "pseudomomentum":
+            w.velocities = rp.PseudomomentumVelocities()
+        return w.model("fp64")
+
+    def calls(m, out):
+        lib, total = m._lib, torch.empty(1, dtype=torch.float64, device="cuda")
+        field = torch.empty(4, 64, dtype=torch.float64, device="cuda")
+        ptrs = [ctypes.c_void_p(field[k].data_ptr()) for k in range(4)] + [ctypes.c_void_p(total.data_ptr())]
+        go.wait()
+        for _ in range(1500):
+            st = (lib.rpl_diagnostics_device(m.handle, *ptrs) if kind == "diagnostics"
+                  else lib.rpl_stage_rows_async(m.handle, 1e-6, 1, 0, 0, 1))   # the stage's preparation alone
+            if st != _lib.RPL_OK:
+                out.append(lib.rpl_last_error().decode())
+                break
+        _lib.check(lib.rpl_sync(m.handle))
+
+    models, errors, go = [make(16), make(120)], [], threading.Barrier(2)
+    threads = [threading.Thread(target=calls, args=(m, errors)) for m in models]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert errors == []
