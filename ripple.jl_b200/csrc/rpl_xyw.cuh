@@ -267,7 +267,10 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
                 }
             }
         }
-        if (!row) return false;
+        if (!row) {   // the CTA does not end with the last row's copies, which nothing reads, in flight
+            if constexpr (ASYNC) copy_wait<0>();
+            return false;
+        }
         if constexpr (XMIX)
             if (act) sg[((1 - buf) * (CX + 1) + slot) * L + l] = own ? codeq(ux1) : 0;   // for the next row
         if constexpr (FUSED) pend(js + k);

@@ -148,3 +148,33 @@ def test_models_of_different_sizes_launch_from_two_threads(kind):
     for t in threads:
         t.join()
     assert errors == []
+
+
+def uneven_depth(shape):
+    x, y = np.meshgrid(np.arange(shape[0]), np.arange(shape[1]), indexing="ij")
+    return np.asfortranarray(2.0 + 0.7 * np.sin(2 * np.pi * x / shape[0]) * np.cos(2 * np.pi * y / shape[1]))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(3, 5, 4, 3), (31, 6, 32, 4), (64, 130, 8, 5), (90, 40, 24, 3), (13, 9, 25, 5), (9, 7, 3, 4),
+                                   (21, 6, 36, 3)])
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+def test_uneven_depth_and_row_ranges(oracle_mod, shape, precision, transport):
+    """c_g per cell, whole and ragged lane vectors, one and several x tiles and segments: the oracle's result, the same
+    bits on every run, and the same bits from stages launched in ranges of one row upwards (the last row of a range is
+    the last its CTA prepares for)."""
+    w = workload(shape, 0.3, None, transport)
+    w.depth = uneven_depth(shape)
+    first = run(w, precision)
+    assert rel_l2(first, oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL[precision]
+    for _ in range(3):
+        assert np.array_equal(run(w, precision), first)
+    m, Ny = w.model(precision), shape[1]
+    cuts = sorted({0, 1, 2, Ny // 2, Ny - 1, Ny})
+    for _ in range(3):
+        for stage in (1, 2, 3):
+            for a, b in zip(cuts[:-1], cuts[1:]):
+                flags = (1 if a == 0 else 0) | (2 if b == Ny else 0)
+                _lib.check(m._lib.rpl_stage_rows_async(m.handle, w.dt, stage, a, b - a, flags))
+    _lib.check(m._lib.rpl_sync(m.handle))
+    assert np.array_equal(m.action.interior(), first)
