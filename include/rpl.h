@@ -203,7 +203,9 @@ typedef struct rpl_source_term {
  * rpl_set_sources (the bundle's tendency comes first). Fields are copied. */
 int rpl_set_source_terms(rpl_handle* h, const rpl_source_term* terms, int32_t count);
 
-/* Replaces set!(model, N=array) / set!(::ProductField, ::AbstractArray) (set.jl:20-30,44-48). */
+/* Replaces set!(model, N=array) / set!(::ProductField, ::AbstractArray) (set.jl:20-30,44-48). The transport's
+ * smoothness indicators square the action and its weights take their square again: steps hold their accuracy
+ * for |N| up to about 1e75 (RPL_FP64) and 1e8 (RPL_FP32); far above, they end in RPL_ERR_DEVICE. */
 int rpl_set_action(rpl_handle* h, const void* N, int32_t dtype, int32_t layout);
 /* Replaces interior(model.action) (product_field.jl:232-235). */
 int rpl_get_action(rpl_handle* h, void* N, int32_t dtype, int32_t layout);

@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "rpl_flux.cuh"
 #include "rpl_src64.cuh"
 #include "rpl_vec.cuh"
 #include "rpl_walk.h"
@@ -263,17 +264,59 @@ struct Lane {
     }
 };
 
+// Stores the lane's result. FP64: a result that is not finite though the action is comes from a face out of weno_face's
+// range, or from a state that blows up; it goes into S (Nout itself, or free) as a mark, so that N0 stays
+// for redo, and *marked is set.
+template <bool AL, typename T, class V>
+__device__ __forceinline__ void store_result(const WalkArgs<T>& p, const Lane<T>& me, V c, V out, int64_t off, int* marked) {
+    if (qfinite(out)) {
+        stv<AL>(p.Nout + off, out, me.left);
+        return;
+    }
+    const bool again = std::is_same<T, double>::value && qfinite(c);
+    if (again) *marked = 1;
+    else atomicOr(p.err, 1u);
+    stv<AL>((again ? p.S : p.Nout) + off, out, me.left);
+}
+
+// The lane's marked results once more, from the tendency of the wider range: after the walk and out of line (inside it,
+// with the walk's registers live, it cost 12% of a refraction and 33% of an intrinsic stage).
+template <bool AL, bool REFRACT, bool BUNDLE>
+__device__ __noinline__ void redo(const WalkArgs<double>& p, const StageParams& sp, int per_part) {
+    const Lane<double> me(p);
+    const int left = me.left, n0 = blockIdx.y * per_part, n1 = min(n0 + per_part, p.Np);
+    Cell64 wc;
+    Bin64 wb[2];
+    if constexpr (BUNDLE) {
+        wc = make_cell64(sp, me.cell);
+        for (int q = 0; q < 2; ++q) wb[q] = make_bin64(sp, me.m0 + min(q, left));
+    }
+    for (int n = n0; n < n1; ++n) {
+        const int64_t off = (int64_t)p.Nx * p.Ny * p.Nk * n + me.home;
+        if (qfinite(ldv<AL>(p.S + off, left))) continue;
+        const D c = ldv<AL>(p.Nin + off, left);
+        D G{bin_tendency_wide<REFRACT>(p, me.cell, me.m0, n), bin_tendency_wide<REFRACT>(p, me.cell, me.m0 + min(1, left), n)};
+        if constexpr (BUNDLE) G = add_source(sp, wc, wb, p.cosp[n], p.sinp[n], c, G);
+        if (p.rates) G = qfma(ldv<AL>(p.rates + off, left), c, G);
+        const D out = stage_update<double>(G, c, p.stage == 1 ? D{0., 0.} : ldv<AL>(p.N0 + off, left), p.stage, p.dt, p.a, p.b);
+        if (!qfinite(out)) atomicOr(p.err, 1u);
+        stv<AL>(p.Nout + off, out, left);
+    }
+}
+
 // Shared memory of ring_kernel in 16-byte slots per thread: the window ring twice, then S and N0 of two steps. Behind
 // them the direction table of the CTA's range, TABLE_NP entries (32 KiB) at most.
 constexpr int WIN = 16, SLOTS = WIN + 4, TABLE_NP = 1024;
 
 template <typename T, bool AL, bool BUNDLE, bool RATES>
 __global__ void __launch_bounds__(RTHREADS, BUNDLE ? 2 : 4)
-ring_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
+ring_kernel(const __grid_constant__ WalkArgs<T> p, const __grid_constant__ StageParams sp, int per_part) {
     using LV = LaneVec<T>;
     using V = typename LV::V;
     using Trig = typename Vel<T>::Trig;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_marked[RTHREADS];   // per thread: some of its results are to be made again
+    s_marked[threadIdx.x] = 0;
     V* slot = reinterpret_cast<V*>(smem) + threadIdx.x;
     Trig* trig = reinterpret_cast<Trig*>(smem + SLOTS * RTHREADS * 16);
     const int Nk = p.Nk, Np = p.Np;
@@ -347,13 +390,12 @@ ring_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
         if constexpr (BUNDLE) G = add_source(sp, wc, wb, __ldg(p.cosp + n), __ldg(p.sinp + n), c, G);
         if (RATES) G = qfma(rate, c, G);   // SourceTermSet rates of this stage, state layout
         const V out = stage_update<T>(G, c, p.stage == 1 ? LV::zero() : lds(st + RTHREADS), p.stage, p.dt, p.a, p.b);
-        if (me.live) {
-            if (!qfinite(out)) atomicOr(p.err, 1u);
-            stv<AL>(p.Nout + off, out, left);
-        }
+        if (me.live) store_result<AL>(p, me, c, out, off, &s_marked[threadIdx.x]);
         off += slice;
         b = (b + 1) & 7;
     }
+    if constexpr (std::is_same<T, double>::value)
+        if (s_marked[threadIdx.x]) redo<AL, true, BUNDLE>(p, sp, per_part);
 }
 
 // Second pass of an intrinsic stage with the FP64 source bundle: G = -S, the sources and the stage update. A
@@ -362,10 +404,13 @@ ring_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
 constexpr int DEPTH = 4;
 
 template <typename T, bool AL, bool RATES>
-__global__ void __launch_bounds__(RTHREADS, 4) bundle_kernel(const WalkArgs<T> p, const StageParams sp, int per_part) {
+__global__ void __launch_bounds__(RTHREADS, 4) bundle_kernel(const __grid_constant__ WalkArgs<T> p,
+                                                               const __grid_constant__ StageParams sp, int per_part) {
     using LV = LaneVec<T>;
     using V = typename LV::V;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_marked[RTHREADS];   // per thread: some of its results are to be made again
+    s_marked[threadIdx.x] = 0;
     V* slot = reinterpret_cast<V*>(smem) + threadIdx.x;
     const int64_t slice = (int64_t)p.Nx * p.Ny * p.Nk;
     const Lane<T> me(p);
@@ -395,11 +440,10 @@ __global__ void __launch_bounds__(RTHREADS, 4) bundle_kernel(const WalkArgs<T> p
         V G = add_source(sp, wc, wb, __ldg(p.cosp + n), __ldg(p.sinp + n), c, qneg(lds(s + RTHREADS)));
         if (RATES) G = qfma(ldv<AL>(p.rates + off, left), c, G);
         const V out = stage_update<T>(G, c, p.stage == 1 ? LV::zero() : lds(s + 2 * RTHREADS), p.stage, p.dt, p.a, p.b);
-        if (me.live) {
-            if (!qfinite(out)) atomicOr(p.err, 1u);
-            stv<AL>(p.Nout + off, out, left);
-        }
+        if (me.live) store_result<AL>(p, me, c, out, off, &s_marked[threadIdx.x]);
     }
+    if constexpr (std::is_same<T, double>::value)
+        if (s_marked[threadIdx.x]) redo<AL, false, true>(p, sp, per_part);
 }
 
 template <typename T, bool AL>

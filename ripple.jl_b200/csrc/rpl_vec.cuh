@@ -34,10 +34,12 @@ __device__ __forceinline__ double rcpd(double x) {
 
 // Nonlinear part of one FP64 WENO5 face, the form of weno_face2 (rpl_weno32.cuh: t_k = 4 (eps + beta_k),
 // linear weights times 10) with the three 1/t_k^2 brought to a common denominator: u_0 : u_1 : u_2 =
-// (t1 t2)^2 : (t0 t2)^2 : (t0 t1)^2. One reciprocal per face instead of four; every product stays in range
-// for |N| up to about 1e38 (t^4 at most 1e307, at least (4 eps)^4 = 6e-45).
+// (t1 t2)^2 : (t0 t2)^2 : (t0 t1)^2. One reciprocal per face instead of four. den grows as t^4 (at least (4 eps)^4 =
+// 6e-45) and num as t^4.5, t ~ 30 N^2: where den reaches 2^850 (N from about 1e31; below it num stays under 2^960) the face
+// is a NaN, and the cell-bin's tendency is computed again by bin_tendency (rpl_flux.cuh), whose weights have the
+// range of 1/t^2 (N to about 1e76), by the kernel that finds its result not finite.
 __device__ __forceinline__ double weno_face(double d1, double d2, double d3, double d4, double D1, double D2,
-                                            double D3, double A1, double A2, double A3, double s2) {
+                                            double D3, double A1, double A2, double A3, double s2, int& den_hi) {
     const double G0 = fma(2.0, d2, D1), G1 = d2 + d3, G2 = fma(-2.0, d3, D3);
     const double t0 = fma(G0, G0, A1), t1 = fma(G1, G1, A2), t2 = fma(G2, G2, A3);
     const double p0 = t1 * t2, p1 = t0 * t2, p2 = t0 * t1;
@@ -45,26 +47,46 @@ __device__ __forceinline__ double weno_face(double d1, double d2, double d3, dou
     const double den = fma(3.0, u2, fma(6.0, u1, u0));
     const double w0 = fma(5.0 / 6.0, d2, (-1.0 / 3.0) * d1), e3 = d3 + d3, w1 = e3 + d2, w2 = fma(-0.5, d4, e3);
     const double num = fma(w2, u2, fma(w1, u1, w0 * u0));
+    den_hi = __double2hiint(den);
     return fma(num, rcpd(den), s2);
+}
+__device__ __forceinline__ double in_range(double f, int den_hi) {
+    return __hiloint2double(den_hi < (1023 + 850) << 20 ? __double2hiint(f) : 0x7ff80000, __double2loint(f));
+}
+__device__ __forceinline__ double weno_face(double d1, double d2, double d3, double d4, double D1, double D2,
+                                            double D3, double A1, double A2, double A3, double s2) {
+    int hi;
+    const double f = weno_face(d1, d2, d3, d4, D1, D2, D3, A1, A2, A3, s2, hi);
+    return in_range(f, hi);
 }
 __device__ __forceinline__ double areg(double D) { return fma((13.0 / 3.0) * D, D, 4.0 * RPL_WENO_EPS); }
 
-__device__ __forceinline__ double weno5_1(double s0, double s1, double s2, double s3, double s4) {
+__device__ __forceinline__ double weno5_1(double s0, double s1, double s2, double s3, double s4, int& den_hi) {
     const double d1 = s1 - s0, d2 = s2 - s1, d3 = s3 - s2, d4 = s4 - s3;
     const double D1 = d2 - d1, D2 = d3 - d2, D3 = d4 - d3;
-    return weno_face(d1, d2, d3, d4, D1, D2, D3, areg(D1), areg(D2), areg(D3), s2);
+    return weno_face(d1, d2, d3, d4, D1, D2, D3, areg(D1), areg(D2), areg(D3), s2, den_hi);
 }
-__device__ __forceinline__ D qweno(D s0, D s1, D s2, D s3, D s4) {
-    return {weno5_1(s0.a, s1.a, s2.a, s3.a, s4.a), weno5_1(s0.b, s1.b, s2.b, s3.b, s4.b)};
+__device__ __forceinline__ double weno5_1(double s0, double s1, double s2, double s3, double s4) {
+    int hi;
+    const double f = weno5_1(s0, s1, s2, s3, s4, hi);
+    return in_range(f, hi);
 }
 
 // A'_c of a second difference, and the face from first differences d, second differences E, regularised
 // squares A and the base value (the two halves of qweno, for stencils that slide by one).
 __device__ __forceinline__ D qareg(D x) { return {areg(x.a), areg(x.b)}; }
 __device__ __forceinline__ Q qareg(Q x) { return {areg(x.a), areg(x.b)}; }
+// (D: one NaN marks the vector, whose results are made again together.)
 __device__ __forceinline__ D qface(D d1, D d2, D d3, D d4, D D1, D D2, D D3, D A1, D A2, D A3, D s2) {
-    return {weno_face(d1.a, d2.a, d3.a, d4.a, D1.a, D2.a, D3.a, A1.a, A2.a, A3.a, s2.a),
-            weno_face(d1.b, d2.b, d3.b, d4.b, D1.b, D2.b, D3.b, A1.b, A2.b, A3.b, s2.b)};
+    int ha, hb;
+    const double fa = weno_face(d1.a, d2.a, d3.a, d4.a, D1.a, D2.a, D3.a, A1.a, A2.a, A3.a, s2.a, ha);
+    const double fb = weno_face(d1.b, d2.b, d3.b, d4.b, D1.b, D2.b, D3.b, A1.b, A2.b, A3.b, s2.b, hb);
+    return {in_range(fa, max(ha, hb)), fb};
+}
+__device__ __forceinline__ D qweno(D s0, D s1, D s2, D s3, D s4) {
+    int ha, hb;
+    const double fa = weno5_1(s0.a, s1.a, s2.a, s3.a, s4.a, ha), fb = weno5_1(s0.b, s1.b, s2.b, s3.b, s4.b, hb);
+    return {in_range(fa, max(ha, hb)), fb};
 }
 __device__ __forceinline__ Q qface(Q d1, Q d2, Q d3, Q d4, Q D1, Q D2, Q D3, Q A1, Q A2, Q A3, Q s2) {
     return {weno_face2(d1.a, d2.a, d3.a, d4.a, D1.a, D2.a, D3.a, A1.a, A2.a, A3.a, s2.a),

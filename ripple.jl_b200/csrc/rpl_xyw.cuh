@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "rpl_flux.cuh"
 #include "rpl_vec.cuh"
 #include "rpl_walk.h"
 
@@ -346,7 +347,7 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
 // moves and take 1.03 ms there, but a small grid pays for fetching the longer code: 17.4 against 14.9 us at
 // 64 x 64 x 4 x 16. Bound: the FP64 pipe (60% busy) and the barrier per row.
 template <bool AL, int XM, int YM, int MODE>
-__device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* fsm, D* priv, int* sg, int n,
+__device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* fsm, D* priv, int* sg, int* marked, int n,
                                          int tx, int js, int je) {
     using T = double;
     using LV = LaneVec<T>;
@@ -515,9 +516,15 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
                 V G = qneg(qadd(fx, fy_prev));
                 if (RATES) G = qfma(plr, cv, G);             // SourceTermSet rates of this stage
                 const V o = stage_update<T>(G, cv, pn0, p.stage, p.dt, p.a, p.b);
-                if (own) {
-                    if (!qfinite(o)) atomicOr(p.err, 1u);
-                    stv<AL>(Sn + outoff - rs, o, left);
+                if (own) {   // a result that is not finite is marked in S, as store_result (rpl_ring.cu) does
+                    if (qfinite(o)) {
+                        stv<AL>(Sn + outoff - rs, o, left);
+                    } else {
+                        const bool again = qfinite(cv);
+                        if (again) marked[threadIdx.x] = 1;
+                        else atomicOr(p.err, 1u);
+                        stv<AL>((again ? p.S + slice * n : Sn) + outoff - rs, o, left);
+                    }
                 }
             }
         }
@@ -606,8 +613,26 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
     for (int k = 0; step(k); ++k) {}
 }
 
+// The results of the thread's column that the whole-stage body marked, once more from the tendency of the wider range
+// (redo in rpl_ring.cu).
+template <bool AL>
+__device__ __noinline__ void redo_column(const WalkArgs<double>& p, int n, int tx, int js, int je) {
+    const int l = threadIdx.x % p.L, slot = threadIdx.x / p.L, i = tx * (p.CX - 1) - 1 + slot;   // own cells only
+    const int m0 = 2 * l, left = p.Nk - 1 - m0;
+    for (int j = js; j < je; ++j) {
+        const int64_t cell = (int64_t)j * p.Nx + i, off = ((int64_t)p.Nx * p.Ny * n + cell) * p.Nk + m0;
+        if (qfinite(ldv<AL>(p.S + off, left))) continue;
+        D G = {bin_tendency_wide<false>(p, cell, m0, n), bin_tendency_wide<false>(p, cell, m0 + min(1, left), n)};
+        const D c = ldv<AL>(p.Nin + off, left);
+        if (p.rates) G = qfma(ldv<AL>(p.rates + off, left), c, G);
+        const D o = stage_update<double>(G, c, p.stage == 1 ? D{0., 0.} : ldv<AL>(p.N0 + off, left), p.stage, p.dt, p.a, p.b);
+        if (!qfinite(o)) atomicOr(p.err, 1u);
+        stv<AL>(p.Nout + off, o, left);
+    }
+}
+
 template <typename T, bool AL, int LB, int XM, int YM, int MODE>
-__device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* smem, int* sg, unsigned bar, int n,
+__device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* smem, int* sg, int* marked, unsigned bar, int n,
                                          int tx, int js, int je) {
     if constexpr (std::is_same<T, float>::value) {
         constexpr int ROWV = XTHREADS + 5 * LB;
@@ -616,7 +641,7 @@ __device__ __forceinline__ void run_body(const WalkArgs<T>& p, unsigned char* sm
                                               je);
     } else {
         D* rows = reinterpret_cast<D*>(smem);
-        xyw_body<AL, XM, YM, MODE>(p, rows, rows + 2 * ROWV64, rows + 2 * ROWV64 + 4 * XTHREADS, sg, n, tx, js, je);
+        xyw_body<AL, XM, YM, MODE>(p, rows, rows + 2 * ROWV64, rows + 2 * ROWV64 + 4 * XTHREADS, sg, marked, n, tx, js, je);
     }
 }
 
@@ -631,10 +656,14 @@ template <typename T, int LB> constexpr size_t xyw_smem() {
 // LB: most lanes per cell the staged rows have room for.
 template <typename T, bool AL, int LB, int MODE>
 __global__ void __launch_bounds__(XTHREADS, 2)
-xyw_kernel(const WalkArgs<T> p, int seg0) {
+xyw_kernel(const __grid_constant__ WalkArgs<T> p, int seg0) {
     constexpr int N = LaneVec<T>::N;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sg[2 * (XTHREADS + MAXL)];
+    // FP64 whole stage, per thread: some of its results are to be made again
+    constexpr bool MARKS = std::is_same<T, double>::value && MODE >= STAGE;
+    __shared__ int marked[MARKS ? XTHREADS : 1];
+    if (MARKS) marked[threadIdx.x] = 0;
     __shared__ __align__(8) unsigned long long row_bar;
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&row_bar);
     if (std::is_same<T, float>::value && threadIdx.x == 0)
@@ -670,17 +699,19 @@ xyw_kernel(const WalkArgs<T> p, int seg0) {
     // component's sign depends on the current. Against the four uniform bodies and one general body: 407 against
     // 431 us per stage at 389 x 251 x 25 x 24 FP32, 1041 against 1068 at 320 x 320 x 32 x 36 FP64.
 #define RPL_BODY(X, Y) \
-    if (xm == X && ym == Y) return run_body<T, AL, LB, X, Y, MODE>(p, smem, sg, bar, n, tx, js, je)
+    if (xm == X && ym == Y) run_body<T, AL, LB, X, Y, MODE>(p, smem, sg, marked, bar, n, tx, js, je)
     RPL_BODY(POS, POS);
-    RPL_BODY(POS, NEG);
-    RPL_BODY(NEG, POS);
-    RPL_BODY(NEG, NEG);
-    RPL_BODY(POS, MIX);
-    RPL_BODY(NEG, MIX);
-    RPL_BODY(MIX, POS);
-    RPL_BODY(MIX, NEG);
-    RPL_BODY(MIX, MIX);
+    else RPL_BODY(POS, NEG);
+    else RPL_BODY(NEG, POS);
+    else RPL_BODY(NEG, NEG);
+    else RPL_BODY(POS, MIX);
+    else RPL_BODY(NEG, MIX);
+    else RPL_BODY(MIX, POS);
+    else RPL_BODY(MIX, NEG);
+    else RPL_BODY(MIX, MIX);
 #undef RPL_BODY
+    if constexpr (MARKS)
+        if (marked[threadIdx.x]) redo_column<AL>(p, n, tx, js, je);
 }
 
 template <typename T, bool AL, int LB, int MODE>

@@ -178,3 +178,28 @@ def test_uneven_depth_and_row_ranges(oracle_mod, shape, precision, transport):
                 _lib.check(m._lib.rpl_stage_rows_async(m.handle, w.dt, stage, a, b - a, flags))
     _lib.check(m._lib.rpl_sync(m.handle))
     assert np.array_equal(m.action.interior(), first)
+
+
+@pytest.mark.parametrize("Nk", [7, 8])
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+def test_large_fp32_action(oracle_mod, Nk, transport):
+    w = workload((11, 8, Nk, 6), 0.3, None, transport)
+    w.N0 = np.asfortranarray(1e8 * w.N0)
+    assert rel_l2(run(w, "fp32"), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL["fp32"]
+
+
+@pytest.mark.parametrize("scale", [1e20, 1e31, 1e36, 1e38, 1e60, 1e75])
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+@pytest.mark.parametrize("sources", ["none", "wind", "linear"])
+def test_large_fp64_action(oracle_mod, scale, transport, sources):
+    """WENO5 weights of large actions (the action enters the smoothness indicators squared and the weights to the fourth
+    power): the oracle's result up to where its own weights end, from everywhere large and from single large cells."""
+    src = {"none": None, "wind": rp.PrecomputedSources(wind_input=rp.PressureCorrelationInput(drag=rp.BulkWindDrag("linear"), wind=18.0,
+                                                                                direction=0.7)),
+           "linear": rp.SourceTermSet(rp.ExponentialWindInput(rate=2e-3, direction=0.6, spreading_power=2))}[sources]
+    for shape in [(11, 8, 7, 6), (9, 12, 8, 5)]:
+        w = workload(shape, 0.3, src, transport)
+        for cells in (1.0, 0.05):
+            large = np.random.default_rng(7).uniform(size=shape) < cells
+            w.N0 = np.asfortranarray(np.where(large, scale, 1.0) * workload(shape).N0)
+            assert rel_l2(run(w, "fp64"), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL["fp64"]
