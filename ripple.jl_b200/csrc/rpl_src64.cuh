@@ -51,7 +51,8 @@ __device__ __forceinline__ Bin64 make_bin64(const StageParams& p, int m) {
     return b;
 }
 
-// Janssen growth rate before the cap; 0 outside the growth window.
+// Janssen growth rate before the cap; 0 outside the growth window and where the parameters make it negative (the
+// reference takes positive rates only).
 __device__ __forceinline__ double wind_rate64(const StageParams& p, const Cell64& c, const Bin64& b, double cth,
                                               double sth) {
     const double cos_tu = fma(cth, c.cu, sth * c.su);
@@ -61,8 +62,9 @@ __device__ __forceinline__ double wind_rate64(const StageParams& p, const Cell64
     if (!(Z < 0.0)) return 0.0;
     const double Z2 = Z * Z;
     const double cp = (p.p_in == 2.0) ? cos_tu * cos_tu : pow(cos_tu, p.p_in);
-    return p.rho_ratio * (p.beta_max / (p.von_karman * p.von_karman)) * exp(Z) * (Z2 * Z2) * (inv_age * inv_age) * cp *
-           b.sigma;
+    const double rate = p.rho_ratio * (p.beta_max / (p.von_karman * p.von_karman)) * exp(Z) * (Z2 * Z2) *
+                        (inv_age * inv_age) * cp * b.sigma;
+    return rate > 0.0 ? rate : 0.0;
 }
 
 // Source tendency of one cell-bin with action a.

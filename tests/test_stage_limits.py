@@ -203,3 +203,15 @@ def test_large_fp64_action(oracle_mod, scale, transport, sources):
             large = np.random.default_rng(7).uniform(size=shape) < cells
             w.N0 = np.asfortranarray(np.where(large, scale, 1.0) * workload(shape).N0)
             assert rel_l2(run(w, "fp64"), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL["fp64"]
+
+
+@pytest.mark.parametrize("precision,Nk", [("fp64", 7), ("fp64", 8), ("fp32", 7)])
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+@pytest.mark.parametrize("parameters", [dict(beta_max=-1.2e3), dict(rho_air=-1.225e3)])
+def test_negative_growth_rates_are_left_out(oracle_mod, precision, Nk, transport, parameters):
+    """Only a positive raw growth rate acts (precomputed_sources.jl:396-439), and only such rates enter the stress."""
+    src = rp.PrecomputedSources(
+        wind_input=rp.PressureCorrelationInput(drag=rp.BulkWindDrag("linear"), wind=18.0, direction=0.7, **parameters),
+        dissipation=rp.LocalSaturationDissipation(B_r=1.05e-2))
+    w = workload((9, 6, Nk, 12), 0.3, src, transport)
+    assert rel_l2(run(w, precision), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL[precision]
