@@ -52,11 +52,13 @@ __device__ __forceinline__ float wind_rate32(const P& p, const Cell32& c, const 
 }
 
 // Whether bin b of cell c can grow in any direction: Z falls with cos(theta - theta_u), so it is positive in every
-// direction where it is at cos = 1 (the margin covers the roundings). Away from a storm no bin can, and the
-// growth rate's exponential and division are skipped there.
+// direction where it is at cos = 1 (the margin covers the roundings); with a negative inverse wave age (z_alpha
+// below -u* / C) it rises, and nothing is left out. Away from a storm no bin can, and the growth rate's exponential
+// and division are skipped there.
 template <class P>
 __device__ __forceinline__ bool can_grow32(const P& p, const Cell32& c, const Bin32& b) {
-    return c.on > 0.5f && (b.logk + c.logz1) + p.von_karman32 / fmaf(c.ustar, b.invC, p.z_alpha32) < 1e-3f;
+    const float inv_age = fmaf(c.ustar, b.invC, p.z_alpha32);
+    return c.on > 0.5f && (inv_age < 0.0f || (b.logk + c.logz1) + p.von_karman32 / inv_age < 1e-3f);
 }
 
 // Source tendency of one cell-bin with action a: wind growth (stress-capped) minus whitecapping. `grows`: the

@@ -215,3 +215,17 @@ def test_negative_growth_rates_are_left_out(oracle_mod, precision, Nk, transport
         dissipation=rp.LocalSaturationDissipation(B_r=1.05e-2))
     w = workload((9, 6, Nk, 12), 0.3, src, transport)
     assert rel_l2(run(w, precision), oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]) <= TOL[precision]
+
+
+@pytest.mark.parametrize("transport", ["refraction", "intrinsic"])
+def test_growth_beside_a_negative_inverse_wave_age(oracle_mod, transport):
+    """z_alpha below -u* / C and a rough surface: log(k z1) > 0, so a bin grows only where cos(theta - theta_u) is small."""
+    src = rp.PrecomputedSources(wind_input=rp.PressureCorrelationInput(
+        drag=rp.BulkWindDrag("linear"), wind=18.0, direction=0.7, z_alpha=-1.0, alpha0=1e4, beta_max=1e4))
+    w = workload((9, 6, 8, 96), 0.3, src, transport)
+    w.dt = 5e-3
+    ref = oracle_mod.Oracle(w).step(w.N0, w.dt, 3)[0]
+    still = workload((9, 6, 8, 96), 0.3, None, transport)
+    still.dt = w.dt
+    assert rel_l2(oracle_mod.Oracle(still).step(w.N0, w.dt, 3)[0], ref) > 10 * TOL["fp32"]     # something grows
+    assert rel_l2(run(w, "fp32"), ref) <= TOL["fp32"]
