@@ -23,8 +23,10 @@ __device__ __forceinline__ Q qfma(Q x, Q y, Q z) { return {fma2(x.a, y.a, z.a), 
 __device__ __forceinline__ D qneg(D x) { return {-x.a, -x.b}; }
 __device__ __forceinline__ Q qneg(Q x) { return {mul2(f2(-1.f), x.a), mul2(f2(-1.f), x.b)}; }
 
-// Reciprocal of a positive normal x: the hardware approximation (about 20 bits) and one third-order step,
-// r (1 + e + e^2) with e = 1 - x r, which leaves e^3 (below 2^-58) before the roundings.
+// Reciprocal of a positive normal x below 2^1022: the hardware approximation (about 20 bits) and one step of
+// Householder's iteration of order two for 1/x (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
+// 1970; for a simple zero also called Chebyshev's iteration), r (1 + e + e^2) with e = 1 - x r, which leaves e^3
+// (below 2^-58) before the roundings. Within one unit in the last place of the correctly rounded quotient.
 __device__ __forceinline__ double rcpd(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
