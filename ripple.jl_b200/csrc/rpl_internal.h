@@ -182,6 +182,7 @@ struct Handle {
     // propagation_smoothing = SpatialAveraging (rpl_smooth.cu)
     bool smooth = false;
     double smooth_as = 0.5, smooth_an = 0.5, smooth_dt = -1.0;  // dt of the current per-bin stencils
+    bool smooth_far = false;       // some bin of that dt may have a corner beyond one cell
     void* d_smooth = nullptr;      // FP64 cg[Nk], dcg[Nk], cos[Np], sin[Np]; per-bin 3x3 stencils; far flags
     int64_t smooth_bytes = 0;
     // snapshot export (rpl_output.cu)

@@ -5,12 +5,12 @@
 // Each spectral bin's physical field is replaced by the mean of four bilinear interpolations at the
 // corners of a rectangle of half-widths L_s = alpha_s |dc_g| dt along the bin's direction and
 // L_n = alpha_n c_g dphi dt across it. When the smoothing is on, the RK3 stage 3 writes its result into
-// the free stage buffer A and smooth_kernel writes A -> N, so the step needs no extra copy and the
+// the free stage buffer A and the averaging kernel writes A -> N, so the step needs no extra copy and the
 // state pointers never change (a captured step stays valid).
 //
 // When every corner lies within one cell of its target (any step that respects the CFL limit), the
 // four samples form a 3 x 3 stencil whose weights depend on the bin only: smooth_weights_kernel builds
-// them once per dt, and smooth_kernel walks strips of cells along x with the 3 x 3 neighbourhood in
+// them once per dt, and smooth_vec_kernel or smooth_kernel walks strips of cells along x with the 3 x 3 neighbourhood in
 // registers (three new kappa-contiguous loads and nine FMAs per output); HBM sees about one read and
 // one write of the state (the neighbouring rows come from L2). Bins whose corners reach further take the
 // reference's per-corner bilinear path. Corner positions are FP64 for both precisions.
@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "rpl_internal.h"
@@ -28,8 +29,8 @@ namespace rpl {
 
 namespace {
 
-constexpr int STRIP = 32;      // cells along x per thread
-constexpr int STHREADS = 192;  // threads per block: whole rows of L lanes
+constexpr int STRIP = 32;      // most cells along x per thread
+constexpr int VTHREADS = 192, STHREADS = 256;  // threads per block of the two averaging kernels
 
 // 1-based index wrap like the reference (_gse_periodic / _gse_clamp), then a clamp so a corner beyond
 // one period never leaves the array.
@@ -118,88 +119,152 @@ __device__ __forceinline__ T sample_far(const T* base, const Corners& k, int i, 
     return acc / T(4);
 }
 
-// Grid (x strips, row groups, directions). A thread walks a strip of STRIP cells along x with one 16-byte vector of
-// adjacent kappa bins (four FP32 or two FP64; L = ceil(Nk / bins) threads per row up to 24, so every thread of
-// a block works whatever Nk is), the 3 x 3 neighbourhood in registers: three vector loads, nine FMAs per bin and one
-// vector store per output. A lane with a far bin (a corner beyond one cell) takes its bins one by one, those
-// through the reference's four bilinear samples. 601 x 417 x 24 x 24 FP32: 613 us with one bin per lane of a
-// 32-lane row; one read and one write of the state are 180 us.
-template <typename T, bool AL>
-__global__ void __launch_bounds__(STHREADS)
-smooth_kernel(const T* __restrict__ Nin, T* __restrict__ Nout, int Nx, int Ny, int Nk, int Np, int L,
-              const T* __restrict__ W, const int* __restrict__ flag, const double* __restrict__ tab, double dphi,
-              double as, double an, double dt, double dx_inv, double dy_inv, int periodic_x, int periodic_y,
-              int j_lo, int j_hi, int y_offset) {
+// What the averaging kernels share. Grid: x strips, bands of rows, directions; a block holds whole rows of L lanes over
+// kappa, so that every thread works whatever Nk is, and a thread walks a strip of cells along x.
+template <typename T>
+struct SmoothArgs {
+    const T* Nin;
+    T* Nout;
+    const T* W;
+    const int* flag;
+    const double* tab;
+    double dphi, as, an, dt, dx_inv, dy_inv;
+    int Nx, Ny, Nk, Np, L, strip, periodic_x, periodic_y, j_lo, j_hi, y_offset;
+};
+
+// The lane's row (1-based like the reference, rows [j_lo, j_hi)) and strip, and the rows of its 3 x 3 neighbourhood.
+template <typename T>
+struct Strip {
+    int l, j, i_first, i_last, n;
+    bool live;
+    const T* base;
+    T* out;
+    int64_t rowoff[3];
+    __device__ __forceinline__ explicit Strip(const SmoothArgs<T>& p) {
+        const int rows = blockDim.x / p.L, row = threadIdx.x / p.L;
+        l = threadIdx.x % p.L;
+        j = p.j_lo + blockIdx.y * rows + row + 1;
+        live = row < rows && j <= p.j_hi;
+        n = blockIdx.z;
+        i_first = blockIdx.x * p.strip + 1;
+        i_last = min(i_first + p.strip - 1, p.Nx);
+        const int64_t P = (int64_t)p.Nx * p.Ny;
+        base = p.Nin + (int64_t)n * P * p.Nk;
+        out = p.Nout + (int64_t)n * P * p.Nk;
+        const int jm = gse_index(j - 1, p.Ny, p.periodic_y), jp = gse_index(j + 1, p.Ny, p.periodic_y);
+        rowoff[0] = (int64_t)(jm - 1) * p.Nx * p.Nk;
+        rowoff[1] = (int64_t)(j - 1) * p.Nx * p.Nk;
+        rowoff[2] = (int64_t)(jp - 1) * p.Nx * p.Nk;
+    }
+};
+
+// FP32 with whole vectors of four kappa bins per lane, where none of the four is far: the 3 x 3 neighbourhood in
+// registers, three 16-byte loads, nine FMAs per bin and one 16-byte store per output. 601 x 417 x 24 x 24: 613 us with one bin
+// per lane of a 32-lane row; one read and one write of the state are 180 us.
+__global__ void __launch_bounds__(VTHREADS) smooth_vec_kernel(const SmoothArgs<float> p) {
     using namespace w32;
-    using LV = LaneVec<T>;
-    using V = typename LV::V;
-    const int rows = STHREADS / L, l = threadIdx.x % L, row = threadIdx.x / L;
-    const int j = j_lo + blockIdx.y * rows + row + 1;  // 1-based like the reference, rows [j_lo, j_hi)
-    if (row >= rows || j > j_hi) return;
-    const int n = blockIdx.z;
-    const int i_first = blockIdx.x * STRIP + 1, i_last = min(i_first + STRIP - 1, Nx);
-    const int64_t P = (int64_t)Nx * Ny;
-    const T* base = Nin + (int64_t)n * P * Nk;
-    T* out = Nout + (int64_t)n * P * Nk;
-    const int jm = gse_index(j - 1, Ny, periodic_y), jp = gse_index(j + 1, Ny, periodic_y);
-    const int64_t rowoff[3] = {(int64_t)(jm - 1) * Nx * Nk, (int64_t)(j - 1) * Nx * Nk, (int64_t)(jp - 1) * Nx * Nk};
-    for (int m0 = l * LV::N; m0 < Nk; m0 += L * LV::N) {
-        const int left = Nk - 1 - m0;
-        bool far = false;
+    const Strip<float> s(p);
+    if (!s.live) return;
+    const int Nk = p.Nk;
+    for (int m0 = 4 * s.l; m0 < Nk; m0 += 4 * p.L) {
+        const int4 far = *reinterpret_cast<const int4*>(p.flag + s.n * Nk + m0);
+        if (far.x | far.y | far.z | far.w) continue;   // the other kernels'
+        Q w[9];
 #pragma unroll
-        for (int q = 0; q < LV::N; ++q) far = far || flag[n * Nk + m0 + min(q, left)];
-        if (far) {
-            for (int m = m0; m <= min(m0 + LV::N - 1, Nk - 1); ++m) {
-                const bool fm = flag[n * Nk + m];
-                const Corners k = corners(tab, Nk, Np, m, n, dphi, as, an, dt, dx_inv, dy_inv);
-                for (int i = i_first; i <= i_last; ++i) {
-                    T acc;
-                    if (fm) {
-                        acc = sample_far(base, k, i, j, m, Nx, Ny, Nk, periodic_x, periodic_y, y_offset);
-                    } else {
-                        const int c[3] = {gse_index(i - 1, Nx, periodic_x) - 1, i - 1, gse_index(i + 1, Nx, periodic_x) - 1};
-                        acc = T(0);
-#pragma unroll
-                        for (int b = 0; b < 3; ++b)
-#pragma unroll
-                            for (int a = 0; a < 3; ++a)
-                                acc = fma(__ldg(W + ((int64_t)n * 9 + b * 3 + a) * Nk + m),
-                                          __ldg(base + rowoff[b] + (int64_t)c[a] * Nk + m), acc);
-                    }
-                    out[((int64_t)(j - 1) * Nx + (i - 1)) * Nk + m] = acc;
-                }
-            }
-            continue;
-        }
-        V w[9];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) w[q] = ldgv<AL>(W + ((int64_t)n * 9 + q) * Nk + m0, left);
+        for (int q = 0; q < 9; ++q) w[q] = ldgq(p.W + ((int64_t)s.n * 9 + q) * Nk + m0);
         // window columns: a = 0 (i-1), 1 (i), 2 (i+1); rows b = 0 (j-1), 1 (j), 2 (j+1)
-        V f[3][3];
-        const int cl = gse_index(i_first - 1, Nx, periodic_x) - 1, cc = i_first - 1;
+        Q f[3][3];
+        const int cl = gse_index(s.i_first - 1, p.Nx, p.periodic_x) - 1, cc = s.i_first - 1;
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-            f[b][0] = ldgv<AL>(base + rowoff[b] + (int64_t)cl * Nk + m0, left);
-            f[b][1] = ldgv<AL>(base + rowoff[b] + (int64_t)cc * Nk + m0, left);
+            f[b][0] = ldgq(s.base + s.rowoff[b] + (int64_t)cl * Nk + m0);
+            f[b][1] = ldgq(s.base + s.rowoff[b] + (int64_t)cc * Nk + m0);
         }
-        T* o = out + ((int64_t)(j - 1) * Nx + (i_first - 1)) * Nk + m0;
+        float* o = s.out + ((int64_t)(s.j - 1) * p.Nx + (s.i_first - 1)) * Nk + m0;
 #pragma unroll 3
-        for (int i = i_first; i <= i_last; ++i, o += Nk) {
-            const int64_t cr = (int64_t)(gse_index(i + 1, Nx, periodic_x) - 1) * Nk + m0;
+        for (int i = s.i_first; i <= s.i_last; ++i, o += Nk) {
+            const int64_t cr = (int64_t)(gse_index(i + 1, p.Nx, p.periodic_x) - 1) * Nk + m0;
 #pragma unroll
-            for (int b = 0; b < 3; ++b) f[b][2] = ldgv<AL>(base + rowoff[b] + cr, left);
-            V acc = LV::zero();
+            for (int b = 0; b < 3; ++b) f[b][2] = ldgq(s.base + s.rowoff[b] + cr);
+            Q acc = qz();
 #pragma unroll
             for (int b = 0; b < 3; ++b)
 #pragma unroll
                 for (int a = 0; a < 3; ++a) acc = qfma(w[b * 3 + a], f[b][a], acc);
-            stv<AL>(o, acc, left);
+            stq(o, acc);
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 f[b][0] = f[b][1];
                 f[b][1] = f[b][2];
             }
         }
+    }
+}
+
+// One bin per lane, adjacent lanes adjacent bins: the near bins by the 3 x 3 stencil. FP64, where pairs of bins per lane hold
+// 72 registers of weights and window and leave too few warps (1283 against 926 us at 512 x 512 x 32 x 24), and ragged
+// FP32, where a vector is four scalar loads (689 against 503 us at 512 x 512 x 25 x 24). Bound by the loads in flight:
+// blocks per SM and unrolling are the fastest of 3 to 6 and 3 to 8. GROUP > 1: only the bins of groups of GROUP with a
+// far one (what smooth_vec_kernel leaves).
+template <typename T, int GROUP>
+__global__ void __launch_bounds__(STHREADS, sizeof(T) == 4 ? 5 : 4) smooth_kernel(const SmoothArgs<T> p) {
+    constexpr int UNROLL = sizeof(T) == 4 ? 4 : 8;
+    const Strip<T> s(p);
+    if (!s.live) return;
+    const int Nk = p.Nk, Nx = p.Nx;
+    const int* flag = p.flag + s.n * Nk;
+    for (int m = s.l; m < Nk; m += p.L) {
+        if (flag[m]) continue;   // smooth_far_kernel's
+        if (GROUP > 1) {
+            bool any = false;
+#pragma unroll
+            for (int q = 0; q < GROUP; ++q) any = any || flag[m - m % GROUP + q];
+            if (!any) continue;
+        }
+        T w[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) w[q] = __ldg(p.W + ((int64_t)s.n * 9 + q) * Nk + m);
+        T f[3][3];
+        const int cl = gse_index(s.i_first - 1, Nx, p.periodic_x) - 1, cc = s.i_first - 1;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            f[b][0] = __ldg(s.base + s.rowoff[b] + (int64_t)cl * Nk + m);
+            f[b][1] = __ldg(s.base + s.rowoff[b] + (int64_t)cc * Nk + m);
+        }
+#pragma unroll UNROLL
+        for (int i = s.i_first; i <= s.i_last; ++i) {
+            const int64_t cr = (int64_t)(gse_index(i + 1, Nx, p.periodic_x) - 1) * Nk + m;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) f[b][2] = __ldg(s.base + s.rowoff[b] + cr);
+            T acc = T(0);
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) acc = fma(w[b * 3 + a], f[b][a], acc);
+            s.out[((int64_t)(s.j - 1) * Nx + (i - 1)) * Nk + m] = acc;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                f[b][0] = f[b][1];
+                f[b][1] = f[b][2];
+            }
+        }
+    }
+}
+
+// The far bins, through the reference's four bilinear samples; a kernel of its own, launched where a bin may be far, so that
+// its registers do not cost the others warps (512 x 512 x 24 directions with every bin far: FP32, 32 bins, 3.9 ms; FP64 4.1).
+template <typename T>
+__global__ void __launch_bounds__(STHREADS) smooth_far_kernel(const SmoothArgs<T> p) {
+    const Strip<T> s(p);
+    if (!s.live) return;
+    const int Nk = p.Nk;
+    for (int m = s.l; m < Nk; m += p.L) {
+        if (!p.flag[s.n * Nk + m]) continue;
+        const Corners k = corners(p.tab, Nk, p.Np, m, s.n, p.dphi, p.as, p.an, p.dt, p.dx_inv, p.dy_inv);
+        T* o = s.out + ((int64_t)(s.j - 1) * p.Nx + (s.i_first - 1)) * Nk + m;
+#pragma unroll 2
+        for (int i = s.i_first; i <= s.i_last; ++i, o += Nk)
+            *o = sample_far(s.base, k, i, s.j, m, p.Nx, p.Ny, Nk, p.periodic_x, p.periodic_y, p.y_offset);
     }
 }
 
@@ -223,6 +288,20 @@ std::vector<double> smooth_tables(const Handle& h) {
     return tab;
 }
 
+// Whether some bin may have a corner beyond one cell for this dt (the device's flags decide; the margin covers
+// the roundings of the two).
+bool may_be_far(const Handle& h, const std::vector<double>& tab, double dphi, double dt) {
+    const int64_t Nk = h.desc.Nk, Np = h.desc.Np;
+    for (int64_t n = 0; n < Np; ++n)
+        for (int64_t m = 0; m < Nk; ++m) {
+            const double Ls = h.smooth_as * tab[Nk + m] * dt, Ln = h.smooth_an * tab[m] * dphi * dt;
+            const double cs = std::fabs(tab[2 * Nk + n]), sn = std::fabs(tab[2 * Nk + Np + n]);
+            const double reach = std::max((Ls * cs + Ln * sn) / h.desc.dx, (Ls * sn + Ln * cs) / h.desc.dy);
+            if (!(reach < 1.0 - 1e-9)) return true;
+        }
+    return false;
+}
+
 template <typename T>
 cudaError_t launch_smooth_t(Handle& h, const void* Nin, void* Nout, double dt, int64_t j_lo, int64_t j_hi,
                             int64_t y_offset, cudaStream_t s) {
@@ -237,16 +316,34 @@ cudaError_t launch_smooth_t(Handle& h, const void* Nin, void* Nout, double dt, i
             Nk, Np, tab, dphi, h.smooth_as, h.smooth_an, dt, 1.0 / d.dx, 1.0 / d.dy, W, flag);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
+        h.smooth_far = may_be_far(h, smooth_tables(h), dphi, dt);
         h.smooth_dt = dt;
     }
-    constexpr int VN = w32::LaneVec<T>::N;
-    const int L = std::min((Nk + VN - 1) / VN, STHREADS / 8), rows = STHREADS / L;   // at least 8 rows per block
-    const dim3 grid((unsigned)((d.Nx + STRIP - 1) / STRIP), (unsigned)((j_hi - j_lo + rows - 1) / rows), (unsigned)Np);
-    auto k = Nk % VN == 0 ? smooth_kernel<T, true> : smooth_kernel<T, false>;
-    k<<<grid, STHREADS, 0, s>>>((const T*)Nin, (T*)Nout, (int)d.Nx, (int)d.Ny, Nk, Np, L, W, flag, tab, dphi, h.smooth_as,
-                                h.smooth_an, dt, 1.0 / d.dx, 1.0 / d.dy, d.periodic_x, d.periodic_y, (int)j_lo, (int)j_hi,
-                                (int)y_offset);
-    return cudaGetLastError();
+    SmoothArgs<T> a{(const T*)Nin, (T*)Nout, W, flag, tab, dphi, h.smooth_as, h.smooth_an, dt, 1.0 / d.dx, 1.0 / d.dy,
+                    (int)d.Nx, (int)d.Ny, Nk, Np, 0, STRIP, d.periodic_x, d.periodic_y, (int)j_lo, (int)j_hi,
+                    (int)y_offset};
+    auto go = [&](auto k, int threads, int lanes) {
+        // at least eight rows per block; a column of more lanes than that leaves is walked in equal chunks
+        const int most = threads / 8, chunks = (lanes + most - 1) / most;
+        a.L = (lanes + chunks - 1) / chunks;
+        const int64_t rows = threads / a.L, bands = (j_hi - j_lo + rows - 1) / rows;
+        // shorter strips (each reads two more columns) where the grid leaves SMs without eight blocks
+        a.strip = STRIP;
+        while (a.strip > 8 && (d.Nx + a.strip - 1) / a.strip * bands * Np < 8 * 148) a.strip /= 2;
+        const dim3 grid((unsigned)((d.Nx + a.strip - 1) / a.strip), (unsigned)bands, (unsigned)Np);
+        k<<<grid, threads, 0, s>>>(a);
+        return cudaGetLastError();
+    };
+    cudaError_t e = cudaSuccess;
+    bool vectors = false;
+    if constexpr (std::is_same<T, float>::value) {
+        vectors = Nk % 4 == 0;
+        if (vectors) e = go(smooth_vec_kernel, VTHREADS, Nk / 4);
+    }
+    if (e == cudaSuccess && (!vectors || h.smooth_far))
+        e = vectors ? go(smooth_kernel<T, 4>, STHREADS, Nk) : go(smooth_kernel<T, 1>, STHREADS, Nk);
+    if (e == cudaSuccess && h.smooth_far) e = go(smooth_far_kernel<T>, STHREADS, Nk);
+    return e;
 }
 
 }  // namespace
