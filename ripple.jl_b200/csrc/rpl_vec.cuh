@@ -90,6 +90,10 @@ __device__ __forceinline__ D qweno(D s0, D s1, D s2, D s3, D s4) {
     const double fa = weno5_1(s0.a, s1.a, s2.a, s3.a, s4.a, ha), fb = weno5_1(s0.b, s1.b, s2.b, s3.b, s4.b, hb);
     return {in_range(fa, max(ha, hb)), fb};
 }
+// A candidate from which elements are selected one by one: each element marks itself.
+__device__ __forceinline__ D qweno_each(D s0, D s1, D s2, D s3, D s4) {
+    return {weno5_1(s0.a, s1.a, s2.a, s3.a, s4.a), weno5_1(s0.b, s1.b, s2.b, s3.b, s4.b)};
+}
 __device__ __forceinline__ Q qface(Q d1, Q d2, Q d3, Q d4, Q D1, Q D2, Q D3, Q A1, Q A2, Q A3, Q s2) {
     return {weno_face2(d1.a, d2.a, d3.a, d4.a, D1.a, D2.a, D3.a, A1.a, A2.a, A3.a, s2.a),
             weno_face2(d1.b, d2.b, d3.b, d4.b, D1.b, D2.b, D3.b, A1.b, A2.b, A3.b, s2.b)};

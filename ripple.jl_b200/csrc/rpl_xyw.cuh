@@ -84,12 +84,12 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
                                               int n, int tx, int js, int je) {
     using LV = LaneVec<float>;
     constexpr bool XMIX = XM == MIX, FUSED = MODE >= STAGE, RATES = MODE == STAGE_RATES, curr = MODE == PASS_CURRENTS;
-    // whole vectors, no currents: rows and c_g by cp.async (874 against 966 us per stage with the SourceTermSet
-    // rates at 384 x 384 x 32 x 36, 704 against 734 without at 601 x 417 x 24 x 24; with currents 1040 against 996
+    // whole vectors, no currents: rows and c_g by cp.async (882 against 962 us per stage with the SourceTermSet
+    // rates at 384 x 384 x 32 x 36, 716 against 739 without at 601 x 417 x 24 x 24; with currents 1040 against 996
     // at 448 x 448, element by element 542 against 418)
     constexpr bool ASYNC = AL && !curr;
     // Rows divided by row_arrive / row_wait: at a barrier a warp stood 0.9 of its 7.4 cycles per instruction.
-    // Against the barrier, cases of 384 x 384 to 1024 x 1024 x 32 x 36: three steps with SourceTermSet rates 8.42 -> 8.06 ms,
+    // Against the barrier, cases of 384 x 384 to 1024 x 1024 x 32 x 36: two steps with SourceTermSet rates 8.42 -> 8.06 ms,
     // tides at 448 x 448 7.48 -> 7.28, self-coupled 11.53 -> 11.2, 1024 x 1024 64.1 -> 63.1; 64 x 64 x 4 x 16, one
     // step, 112 -> 114 us (latency). Vectors copied element by element keep the barrier: 7.68 against 7.92 ms
     // at 389 x 251 x 25 x 24.
@@ -345,7 +345,8 @@ __device__ __forceinline__ void xyw_body_ring(const WalkArgs<float>& p, Q* ring,
 // order, so a spilled value then waited for the row's loads from DRAM (1.30 against 1.07 ms per stage at
 // 320 x 320 x 32 x 36). Four copies of the step with the stencil in rings indexed at compile time need no
 // moves and take 1.03 ms there, but a small grid pays for fetching the longer code: 17.4 against 14.9 us at
-// 64 x 64 x 4 x 16. Bound: the FP64 pipe (60% busy) and the barrier per row.
+// 64 x 64 x 4 x 16. Bound: the FP64 pipe (55% busy with currents, 57%
+// without), issue (62%) and the barrier per row.
 template <bool AL, int XM, int YM, int MODE>
 __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* fsm, D* priv, int* sg, int* marked, int n,
                                          int tx, int js, int je) {
@@ -430,8 +431,8 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
         for (int d = -2; d <= 3; ++d) w[d + 2] = ld(modr(js + d), colm);
         const V below = ld(modr(js - 3), colm);
         const int need = own ? codeq(uy0) : 0;
-        if (__any_sync(FULL, need & 1)) pLy = qweno(below, w[0], w[1], w[2], w[3]);
-        if (__any_sync(FULL, need & 2)) pRy = qweno(w[4], w[3], w[2], w[1], w[0]);
+        if (__any_sync(FULL, need & 1)) pLy = qweno_each(below, w[0], w[1], w[2], w[3]);
+        if (__any_sync(FULL, need & 2)) pRy = qweno_each(w[4], w[3], w[2], w[1], w[0]);
         rload(0, modr(js + 4));
     } else if constexpr (YM == POS) {
         const V r0 = ld(modr(js - 3), colm), r1 = ld(modr(js - 2), colm), r2 = ld(modr(js - 1), colm);
@@ -542,8 +543,8 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
             } else {
                 const int need = (own ? codeq(ux0) : 0) | sg[(buf * (CX + 1) + slot + 1) * L + l];
                 V Lx = LV::zero(), Rx = LV::zero();
-                if (__any_sync(FULL, need & 1)) Lx = qweno(X(-2), X(-1), c, X(1), X(2));
-                if (__any_sync(FULL, need & 2)) Rx = qweno(X(3), X(2), X(1), c, X(-1));
+                if (__any_sync(FULL, need & 1)) Lx = qweno_each(X(-2), X(-1), c, X(1), X(2));
+                if (__any_sync(FULL, need & 2)) Rx = qweno_each(X(3), X(2), X(1), c, X(-1));
                 if (act) {
                     sts(fsm + ((buf * CX + slot) * L + l) * 2, Lx);
                     sts(fsm + ((buf * CX + slot) * L + l) * 2 + 1, Rx);
@@ -557,8 +558,8 @@ __device__ __forceinline__ void xyw_body(const WalkArgs<double>& p, D* rowb, D* 
             if constexpr (YMIX) {
                 const int need = own ? (codeq(uy0) | (k + 1 < cnt ? codeq(uy1) : 0)) : 0;
                 V Ly = LV::zero(), Ry = LV::zero();
-                if (__any_sync(FULL, need & 1)) Ly = qweno(w[0], w[1], w[2], w[3], w[4]);
-                if (__any_sync(FULL, need & 2)) Ry = qweno(w[5], w[4], w[3], w[2], w[1]);
+                if (__any_sync(FULL, need & 1)) Ly = qweno_each(w[0], w[1], w[2], w[3], w[4]);
+                if (__any_sync(FULL, need & 2)) Ry = qweno_each(w[5], w[4], w[3], w[2], w[1]);
                 Fhi = selq(uy0, Ly, Ry);
                 Flo = selq(uy0, pLy, pRy);
                 pLy = Ly;

@@ -229,3 +229,20 @@ def test_growth_beside_a_negative_inverse_wave_age(oracle_mod, transport):
     still.dt = w.dt
     assert rel_l2(oracle_mod.Oracle(still).step(w.N0, w.dt, 3)[0], ref) > 10 * TOL["fp32"]     # something grows
     assert rel_l2(run(w, "fp32"), ref) <= TOL["fp32"]
+
+
+@pytest.mark.parametrize("scale", [3e31, 1e33, 3e33, 1e34, 1e35, 1e37, 3e37])
+def test_large_fp64_action_where_neighbouring_bins_upwind_apart(oracle_mod, scale):
+    """Currents as fast as the waves: the two bins of a lane take their faces from different sides. Large cells in every
+    other bin alone (four bins have no kappa stencil that would join them), so that one bin's face leaves the range on the
+    side its neighbour does not use."""
+    for shape in [(24, 20, 16, 9), (60, 50, 4, 12), (60, 50, 3, 11)]:
+        w = workload(shape, 3.0)
+        rng = np.random.default_rng(11)
+        large = rng.uniform(size=shape) < 0.04
+        if shape[2] < 5:
+            large[:, :, 0::2] = False
+        w.N0 = np.asfortranarray(np.where(large, scale * 10.0 ** rng.uniform(-3, 0, shape), 1.0) * workload(shape).N0)
+        out, ref = run(w, "fp64", 1), oracle_mod.Oracle(w).step(w.N0, w.dt, 1)[0]
+        assert rel_l2(out, ref) <= TOL["fp64"]
+        assert np.array_equal(out == 0.0, ref == 0.0)
