@@ -122,20 +122,17 @@ def make_workload(name, n, nsteps, n0_dtype=np.float64):
 
 
 def launches_per_step(name, precision="fp32"):
-    """Our kernels per RK3 step. A stage is two launches in FP32 (refraction: the x/y flux pass, then the
-    kappa/phi pass with the stage update; the hurricane's intrinsic transport with the bundle sources: the
-    x/y pass, then the sources and the update) and one fused launch in FP64; the hurricane adds 1 wind + 3
-    stress-cap kernels; the self-coupled swell adds 2 coupling kernels per stage, and in FP32 the refresh
-    of the velocity planes of the x/y pass."""
-    per_stage = 2 if precision == "fp32" else 1
-    coupling = 3 if precision == "fp32" else 2
-    return {"seamount": 3 * per_stage, "selfcoupled": 3 * (per_stage + coupling)}.get(name, 3 * per_stage + 4)
+    """Our kernels per RK3 step. A stage is two launches in both precisions (refraction: the x/y flux pass, then
+    the kappa/phi pass with the stage update; the hurricane's intrinsic transport with the bundle sources: the
+    x/y pass, then the sources and the update); the hurricane adds 1 wind + 3 stress-cap kernels; the self-coupled
+    swell adds 3 per stage: the pseudomomentum velocity, the coefficient records and the velocity planes."""
+    return {"seamount": 3 * 2, "selfcoupled": 3 * (2 + 3)}.get(name, 3 * 2 + 4)
 
 
 def current_launches(precision):
-    """Kernels of one update of time-varying currents: Q transform, gradients, coefficient records, and
-    in FP32 the velocity planes of the x/y pass."""
-    return 4 if precision == "fp32" else 3
+    """Kernels of one update of time-varying currents: Q transform, coefficient records (with the gradients) and the
+    velocity planes of the x/y pass."""
+    return 3
 
 
 def peaks():
