@@ -97,7 +97,7 @@ CONFIG_STEPS = {"seamount": 200, "hurricane": 1000, "selfcoupled": 200}   # RK3 
 WORKLOAD_NAMES = {"seamount": "seamount_eddies", "hurricane": "hurricane_swell", "ensemble": "ensemble_members",
                   "learned": "hurricane_swell (learned source)", "selfcoupled": "self_coupled_swell"}
 TRAFFIC_SUFFIX = {"seamount": "", "hurricane": "_hurricane", "selfcoupled": "_selfcoupled"}
-# the FP32 stage kernels each workload runs (refraction: two passes per stage; intrinsic: one fused kernel)
+# the stage kernels each workload runs, two passes per stage (FP64 takes the bundle's sources in bundle_kernel)
 STAGE_KERNELS = {"seamount": "xyw_kernel+ring_kernel", "hurricane": "xyw_kernel+ks_kernel",
                  "selfcoupled": "xyw_kernel+ring_kernel"}
 DATA = {"seamount": "synthetic (seeded seamount depth, eddy currents, JONSWAP-like N0)",
@@ -525,7 +525,7 @@ def run_ours(args, rank, world, local_rank):
                           if snap_bufs is not None else {})},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": STAGE_KERNELS[args.workload] if args.precision == "fp32" else "column_kernel",
+                         "kernel": STAGE_KERNELS[args.workload].replace("ks_kernel", "ks_kernel" if args.precision == "fp32" else "bundle_kernel"),
                          "launch_ms": launch_ms, "algorithmic_bytes_per_launch": bytes_per_launch,
                          "launch_interval": "one RK3 stage" + {"seamount": "",
                                                                "selfcoupled": " incl. its coupling refresh"}.get(
