@@ -133,11 +133,10 @@ struct BinArgs {
     T dx_inv, dy_inv, dk_inv, dp_inv;
 };
 
-// Transport tendency of bin (m, n) of cell c.
+// Transport tendency of bin (m, n) of cell c = i + Nx j, whose action is c0.
 template <typename T, bool REFRACT>
-__device__ __forceinline__ T bin_tendency(const BinArgs<T>& p, int64_t c, int m, int n) {
+__device__ __forceinline__ T bin_tendency(const BinArgs<T>& p, int64_t c, int i, int j, int m, int n, T c0) {
     const int Nx = p.Nx, Ny = p.Ny, Nk = p.Nk, Np = p.Np;
-    const int i = (int)(c % Nx), j = (int)(c / Nx);
     const int64_t slice = (int64_t)Nx * Ny * Nk;
     const Coef q = load_coef(p.coef + 8 * (c * Nk + m));
     const int b = m + Nk * n;
@@ -146,7 +145,6 @@ __device__ __forceinline__ T bin_tendency(const BinArgs<T>& p, int64_t c, int m,
     const T* row = p.N + (int64_t)n * slice;
     auto X = [&](int ii) { return row[((int64_t)j * Nx + wrap(ii, Nx)) * Nk + m]; };
     auto Y = [&](int jj) { return row[((int64_t)wrap(jj, Ny) * Nx + i) * Nk + m]; };
-    const T c0 = row[c * Nk + m];
     const T fx = flux_diff(X(i - 3), X(i - 2), X(i - 1), c0, X(i + 1), X(i + 2), X(i + 3), ux) * p.dx_inv;
     const T fy = flux_diff(Y(j - 3), Y(j - 2), Y(j - 1), c0, Y(j + 1), Y(j + 2), Y(j + 3), uy) * p.dy_inv;
     if constexpr (!REFRACT) return -(fx + fy);
@@ -172,7 +170,8 @@ template <bool REFRACT>
 static __device__ __noinline__ double bin_tendency_wide(const WalkArgs<double>& p, int64_t c, int m, int n) {
     const BinArgs<double> b{p.Nin, p.coef, p.cosp, p.sinp, p.cgx, p.cgy, p.Nx, p.Ny, p.Nk, p.Np, p.cg_per_cell,
                             p.dx_inv, p.dy_inv, p.dk_inv, p.dp_inv};
-    return bin_tendency<double, REFRACT>(b, c, m, n);
+    return bin_tendency<double, REFRACT>(b, c, (int)(c % p.Nx), (int)(c / p.Nx), m, n,
+                                         p.Nin[((int64_t)p.Nx * p.Ny * n + c) * p.Nk + m]);
 }
 
 }  // namespace rpl

@@ -197,12 +197,12 @@ __global__ void __launch_bounds__(BLOCK) generic_kernel(const T* __restrict__ Ni
     const int64_t cn = t / Nk;
     const int64_t c = cn % P;
     const int n = (int)(cn / P);
-    const int j = (int)(c / Nx);
+    const int i = (int)(c % Nx), j = (int)(c / Nx);
     if (j < p.j_lo || j >= p.j_hi) return;
     const BinArgs<T> b{Nin, p.coef, p.cosp, p.sinp, p.cg_x, p.cg_y, Nx, Ny, Nk, Np, p.cg_per_cell,
                        T(p.dx_inv), T(p.dy_inv), T(p.dk_inv), T(p.dp_inv)};
     const T c0 = Nin[t];
-    T G = bin_tendency<T, REFRACT>(b, c, m, n);
+    T G = bin_tendency<T, REFRACT>(b, c, i, j, m, n, c0);
     if (p.has_wind || p.has_diss) G = G + T(source_term(p, c, m, n, (double)c0));
     if (p.lin_rates) G = fma(static_cast<const T*>(p.lin_rates)[t], c0, G);
     if constexpr (TENDENCY) {
