@@ -87,7 +87,7 @@ __global__ void pm_overlap_kernel(int Nk, int64_t Nz, int kc_max, const double* 
 // serves the warp's columns) or one per column. Ux, Uy: c3 doubles each in device order c*Nk + t. A is the
 // arithmetic type: double for FP64 models and for dU/dkappa, float for the per-stage refresh of FP32 models.
 // One column per warp took 243 us at 384 x 384 x 32 x 36 FP32; reading the state once is 105 us.
-template <typename T, typename A, bool AL, bool SMEM>
+template <typename T, typename A>
 __global__ void __launch_bounds__(PM_WARPS * 32)
 pm_velocity_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* __restrict__ kx,
                    const A* __restrict__ ky, const A* __restrict__ O, int per_cell, double* __restrict__ Ux,
@@ -97,14 +97,12 @@ pm_velocity_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* 
     const int warp = threadIdx.x >> 5;
     const int stride = table_stride<T>(Nk), size = stride * Np;
     A* tab = reinterpret_cast<A*>(pm_smem);
-    if constexpr (SMEM) {
-        stage_table(tab, kx, Nk, Np, stride);
-        stage_table(tab + size, ky, Nk, Np, stride);
-        __syncthreads();
-    }
+    stage_table(tab, kx, Nk, Np, stride);
+    stage_table(tab + size, ky, Nk, Np, stride);
+    __syncthreads();
     const ColVec<T> v(Nk);
     // per warp the moments of its columns, x then y: 2 cpw stride
-    A* mom = tab + (SMEM ? 2 * size : 0) + warp * 2 * v.cpw * stride;
+    A* mom = tab + 2 * size + warp * 2 * v.cpw * stride;
     A* mx = mom + v.col() * stride;
     A* my = mx + v.cpw * stride;
     const int64_t slice = P * Nk, groups = (P + v.cpw - 1) / v.cpw;
@@ -113,22 +111,21 @@ pm_velocity_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* 
         __syncwarp();
         for (int m0 = v.l * VN; m0 < Nk; m0 += 32 * VN) {
             const T* p = N + c * Nk + m0;
-            const int left = Nk - 1 - m0;
             A ax[VN] = {}, ay[VN] = {};
             for (int n0 = 0; n0 < Np; n0 += CH, p += CH * slice) {
                 T f[CH][VN];
 #pragma unroll
                 for (int k = 0; k < CH; ++k)
-                    if (n0 + k < Np) ld_bins<AL>(p + k * slice, left, f[k]);
+                    if (n0 + k < Np) ld_bins<true>(p + k * slice, VN - 1, f[k]);
 #pragma unroll
                 for (int k = 0; k < CH; ++k) {
                     if (n0 + k >= Np) break;
 #pragma unroll
                     for (int q = 0; q < VN; ++q) {
-                        const int at = (n0 + k) * stride + m0 + q, gb = (n0 + k) * Nk + m0 + min(q, left);
+                        const int at = (n0 + k) * stride + m0 + q;
                         const A a = (A)f[k][q];
-                        ax[q] += a * (SMEM ? tab[at] : __ldg(kx + gb));
-                        ay[q] += a * (SMEM ? tab[size + at] : __ldg(ky + gb));
+                        ax[q] += a * tab[at];
+                        ay[q] += a * tab[size + at];
                     }
                 }
             }
@@ -143,27 +140,63 @@ pm_velocity_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* 
         __syncwarp();
         const A* o = per_cell ? O + c * (int64_t)Nk * Nk : O;
         for (int t0 = v.l * VN; t0 < Nk; t0 += 32 * VN) {
-            const int left = Nk - 1 - t0;
             A ux[VN] = {}, uy[VN] = {};
 #pragma unroll 4
             for (int s = 0; s < Nk; ++s) {
                 const A px = mx[s], py = my[s];
 #pragma unroll
                 for (int q = 0; q < VN; ++q) {
-                    const A w = __ldg(o + s * Nk + t0 + min(q, left));
+                    const A w = __ldg(o + s * Nk + t0 + q);
                     ux[q] += w * px;
                     uy[q] += w * py;
                 }
             }
             if (v.used && col < P) {
 #pragma unroll
-                for (int q = 0; q < VN; ++q)
-                    if (q <= left) {
-                        Ux[c * Nk + t0 + q] = (double)ux[q];
-                        Uy[c * Nk + t0 + q] = (double)uy[q];
-                    }
+                for (int q = 0; q < VN; ++q) {
+                    Ux[c * Nk + t0 + q] = (double)ux[q];
+                    Uy[c * Nk + t0 + q] = (double)uy[q];
+                }
             }
         }
+    }
+}
+
+// The same with one warp per column and the tables through L1, for any Nk and grid.
+template <typename T, typename A>
+__global__ void __launch_bounds__(PM_WARPS * 32)
+pm_column_kernel(const T* __restrict__ N, int64_t P, int Nk, int Np, const A* __restrict__ kx,
+                   const A* __restrict__ ky, const A* __restrict__ O, int per_cell, double* __restrict__ Ux,
+                   double* __restrict__ Uy) {
+    extern __shared__ __align__(16) unsigned char pm_smem[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * PM_WARPS + w;
+    if (c >= P) return;  // uniform per warp; the kernel has no block-wide barrier
+    A* mx = reinterpret_cast<A*>(pm_smem) + (int64_t)w * 2 * Nk;
+    A* my = mx + Nk;
+    for (int s = lane; s < Nk; s += 32) {
+        A ax = 0, ay = 0;
+#pragma unroll 6
+        for (int n = 0; n < Np; ++n) {
+            const A a = (A)N[((int64_t)n * P + c) * Nk + s];
+            ax += a * __ldg(kx + s + (int64_t)Nk * n);
+            ay += a * __ldg(ky + s + (int64_t)Nk * n);
+        }
+        mx[s] = ax;
+        my[s] = ay;
+    }
+    __syncwarp();
+    const A* o = per_cell ? O + c * (int64_t)Nk * Nk : O;
+    for (int t = lane; t < Nk; t += 32) {
+        A ux = 0, uy = 0;
+#pragma unroll 8
+        for (int s = 0; s < Nk; ++s) {
+            const A q = __ldg(o + (int64_t)s * Nk + t);
+            ux += q * mx[s];
+            uy += q * my[s];
+        }
+        Ux[c * Nk + t] = (double)ux;
+        Uy[c * Nk + t] = (double)uy;
     }
 }
 
@@ -186,13 +219,20 @@ cudaError_t pm_velocity(const Handle& h, const void* Nin, const A* moments, cons
     const int Nk = (int)h.desc.Nk, Np = (int)h.desc.Np;
     const int64_t P = h.cells, c3 = P * Nk, nb = (int64_t)Nk * Np;
     constexpr int VN = ColVec<T>::N;
-    const int stride = table_stride<T>(Nk);
-    const int64_t cpw = 32 / std::min((Nk + VN - 1) / VN, 32);
-    const size_t mom = (size_t)PM_WARPS * 2 * cpw * stride * sizeof(A), tab = 2 * (size_t)stride * Np * sizeof(A);
-    const bool staged = tab + mom <= kTableBytes;
-    auto k = !staged ? pm_velocity_kernel<T, A, false, false>
-                     : (Nk % VN == 0 ? pm_velocity_kernel<T, A, true, true> : pm_velocity_kernel<T, A, false, true>);
-    const size_t smem = mom + (staged ? tab : 0);
+    const int stride = table_stride<T>(Nk), L = std::min((Nk + VN - 1) / VN, 32);
+    const int64_t cpw = 32 / L;
+    const size_t smem = (PM_WARPS * 2 * cpw * stride + 2 * (size_t)stride * Np) * sizeof(A);
+    // Lane vectors where they are whole, fill the warp (several columns, or all lanes with one) and the columns are
+    // many enough to pay for staging the tables in every block; else a warp per column. us per stage with the refresh of
+    // the planes: FP32 384 x 384 x 32 x 36 325 against 401 by columns, 256 x 256 x 25 x 24 160 against 149, 64 x 64 x 100 x 24
+    // 63 against 50, 32 x 32 x 32 x 36 25 against 21; FP64 256 x 256 x 64 x 36 506 against 589, x 40 400 against 364,
+    // 64 x 64 x 100 x 24 94 against 117.
+    if (Nk % VN != 0 || (cpw < 2 && L < 32) || (P < 8192 && P * Nk < 300000) || smem > kTableBytes) {
+        pm_column_kernel<T, A><<<blocks_for(P, PM_WARPS), PM_WARPS * 32, (size_t)PM_WARPS * 2 * Nk * sizeof(A), s>>>(
+            (const T*)Nin, P, Nk, Np, moments, moments + nb, overlap, h.pm_cols > 1, U, U + c3);
+        return cudaGetLastError();
+    }
+    auto k = pm_velocity_kernel<T, A>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)std::min<int64_t>(blocks_for(P, (int)(PM_WARPS * cpw)), 148 * 4);
